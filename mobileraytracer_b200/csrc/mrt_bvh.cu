@@ -5,15 +5,14 @@
 // reorders primitives, so leaf offsets index the input arrays.
 //
 // FAST tree: built on the device.  Triangle boxes padded outward -> 30-bit Morton codes of the
-// centroids -> stable LSD radix sort (own kernels) -> Karras' parallel hierarchy ("Maximizing
-// parallelism in the construction of BVHs, octrees and k-d trees", HPG 2012) -> bottom-up box fit
-// -> records in child-pair layout (32 bytes per record), subtrees of <= leaf_max_setting() (at most 3)
-// triangles collapsed into leaves where the surface-area cost says so -> the binary tree collapsed
-// into 8-wide nodes with 16-bit quantised child boxes (128 bytes: one cache line per traversal step;
-// each wide node opens the largest internal children of a binary node until it holds 8), children
-// placed in slots by octant, internal children numbered consecutively, the leaf children's triangles
-// copied to consecutive 48-byte records.  A traversal step of the 8-wide tree replaces about three of
-// the binary tree's, shortening the chain of dependent node fetches per ray.
+// centroids on a grid of cubes -> stable LSD radix sort (own kernels) -> Karras' parallel hierarchy
+// ("Maximizing parallelism in the construction of BVHs, octrees and k-d trees", HPG 2012) -> bottom-up
+// box fit, which also works out for every binary node the cheapest way to turn its subtree into wide
+// nodes -> the binary tree collapsed along those choices into 8-wide nodes with 16-bit quantised
+// child boxes (128 bytes: one cache line per traversal step), children placed in slots by octant,
+// internal children numbered consecutively, the leaf children's triangles copied to consecutive
+// 48-byte records.  A traversal step of the 8-wide tree replaces about three of the binary tree's,
+// shortening the chain of dependent node fetches per ray.
 #include <algorithm>
 #include <cstdlib>
 #include <cstring>
@@ -157,17 +156,25 @@ __device__ __forceinline__ uint32_t expand_bits(uint32_t v) {   // 10 bits -> ev
     return v;
 }
 
+// Codes on a grid of cubes over the longest side of the centroid bounds, 1024 a side.  (A grid of
+// 1024 cells along every axis whatever its extent cuts flat scenes across their thin axis as often as
+// along the others: on the 524,288-triangle heightfield, 0.35 high over a side of 2, a camera ray then
+// visits 10.9 nodes and a bounce 16.4, with cubes 9.1 and 14.4; scenes as deep as wide keep their codes.)
 __global__ void k_morton(uint32_t n, const float4 *__restrict__ bmin, const float4 *__restrict__ bmax,
                          const uint32_t *__restrict__ cbounds, uint32_t *keys, uint32_t *vals) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 lo = bmin[i], hi = bmax[i];
-    float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
+    const float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
+    float mn[3], ext[3], side = 0.0f;
+    for (int k = 0; k < 3; ++k) {
+        mn[k] = key_float_(cbounds[k]);
+        ext[k] = key_float_(cbounds[3 + k]) - mn[k];
+        if (ext[k] > side && ext[k] <= 3.0e38f) side = ext[k];   // finite sides only
+    }
     uint32_t q[3];
     for (int k = 0; k < 3; ++k) {
-        const float mn = key_float_(cbounds[k]), mx = key_float_(cbounds[3 + k]);
-        const float ext = mx - mn;
-        float u = ext > 0.0f ? (c[k] - mn) / ext : 0.5f;
+        float u = (ext[k] > 0.0f && ext[k] <= 3.0e38f) ? (c[k] - mn[k]) / side : 0.5f;
         u = fminf(fmaxf(u, 0.0f), 1.0f);
         q[k] = min((uint32_t)(u * 1024.0f), 1023u);
     }
@@ -189,31 +196,56 @@ __global__ void k_rs_hist(const uint32_t *__restrict__ keys, uint32_t n, int shi
     hist[threadIdx.x * nblocks + blockIdx.x] = cnt[threadIdx.x];
 }
 
-// exclusive scan of m values in place, one block of 1024 threads
-__global__ void k_scan_exclusive(uint32_t *data, uint32_t m) {
-    __shared__ uint32_t part[1024];
-    const uint32_t per = (m + 1023) / 1024;
-    const uint32_t b = threadIdx.x * per, e = min(b + per, m);
-    uint32_t s = 0;
-    for (uint32_t i = b; i < e; ++i) s += data[i];
-    part[threadIdx.x] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const uint32_t v = threadIdx.x >= (uint32_t)o ? part[threadIdx.x - o] : 0u;
+// exclusive scan of each digit's row of per-block counts in place (one block of 256 threads per
+// digit), the row sums to total[digit]; k_rs_scatter adds the digits before a row.  (One block over
+// all 256 rows took 105 us a pass at 1,000,000 keys, 12 % of the build's kernels; the rows take 3 us.)
+__global__ void __launch_bounds__(256) k_rs_scan_rows(uint32_t *hist, uint32_t nblocks, uint32_t *total) {
+    __shared__ uint32_t wsum[8];
+    uint32_t *row = hist + (size_t)blockIdx.x * nblocks;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = 0;
+    for (uint32_t b = 0; b < nblocks; b += 256) {
+        const uint32_t i = b + threadIdx.x;
+        const uint32_t v = i < nblocks ? row[i] : 0u;
+        uint32_t incl = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += w;
+        }
+        if (lane == 31) wsum[warp] = incl;
         __syncthreads();
-        part[threadIdx.x] += v;
+        uint32_t before = 0, all = 0;
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (i < nblocks) row[i] = carry + before + incl - v;
+        carry += all;
         __syncthreads();
     }
-    uint32_t acc = part[threadIdx.x] - s;
-    for (uint32_t i = b; i < e; ++i) { const uint32_t v = data[i]; data[i] = acc; acc += v; }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
 }
 
 __global__ void k_rs_scatter(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin, uint32_t *kout,
-                             uint32_t *vout, uint32_t n, int shift, const uint32_t *__restrict__ hist, uint32_t nblocks) {
+                             uint32_t *vout, uint32_t n, int shift, const uint32_t *__restrict__ hist, uint32_t nblocks,
+                             const uint32_t *__restrict__ digit_total) {
     __shared__ uint32_t base[256], running[256], total[256];
     __shared__ uint32_t wcnt[kSortThreads / 32][256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    base[tid] = hist[tid * nblocks + blockIdx.x];
+    {   // the keys of smaller digits, then this block's place in its digit's row
+        const uint32_t v = digit_total[tid];
+        uint32_t incl = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += w;
+        }
+        if (lane == 31) total[warp] = incl;
+        __syncthreads();
+        uint32_t before = 0;
+        for (int w = 0; w < warp; ++w) before += total[w];
+        base[tid] = before + incl - v + hist[tid * nblocks + blockIdx.x];
+        __syncthreads();
+    }
     running[tid] = 0;
     const uint32_t lt_mask = (1u << lane) - 1u;
     for (int r = 0; r < kSortItems; ++r) {
@@ -296,168 +328,135 @@ __device__ __forceinline__ void child_box(uint32_t c, const uint32_t *__restrict
     }
 }
 
-__global__ void k_fit(int n, const uint32_t *__restrict__ vals, const float4 *__restrict__ bmin,
+__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
+    const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
+    return dx * dy + dy * dz + dz * dx;
+}
+
+// --- the cheapest wide nodes of every subtree --------------------------------------------------------
+// Ylitie, Karras and Laine, "Efficient Incoherent Ray Traversal on GPUs Through Compressed Wide BVHs"
+// (HPG 2017), section 3.1: C(n, j) = the least surface-area cost of a binary subtree n held in at most j
+// child slots of a wide node, j = 1..7.  One slot holds a leaf of up to leaf_max triangles (kTriCost x
+// triangles x box area) or a wide node of its own (box area x kNodeCost + the best split of 8 slots over
+// n's two children); more slots hold the best split of j over the two children, or fewer of them.  The
+// costs of a node and the choices behind them (one word) are worked out bottom-up in the pass that fits
+// the boxes: 28 additions and comparisons a node.  Against opening the largest child until a node is
+// full, the nodes visited per camera ray go from 24.8 to 23.6 on the 1,000,000-triangle soup (tree
+// 36.4 -> 30 MB) and from 9.1 to 8.8 on the heightfield (14.4 -> 13.8 after a bounce; 12.2 -> 7.9 MB).
+#ifndef MRT_BVH_TRI_COST
+#define MRT_BVH_TRI_COST 0.9f
+#endif
+constexpr float kTriCost = MRT_BVH_TRI_COST, kNodeCost = 1.0f;
+
+struct SlotCosts {      // 32 bytes per binary internal node
+    float c[7];         // C(n, 1..7)
+    uint32_t choice;    // bit 0: one slot holds a leaf; bits 1-3: slots of the left child when n is a wide
+                        // node (of 8); bits 4 + 3 (j - 2)..: slots of the left child out of j (0: as j - 1)
+};
+__device__ __forceinline__ uint32_t choice_node_split(uint32_t choice) { return (choice >> 1) & 7u; }
+__device__ __forceinline__ uint32_t choice_split(uint32_t choice, uint32_t j) { return (choice >> (4u + 3u * (j - 2u))) & 7u; }
+
+__device__ __forceinline__ void child_costs(uint32_t c, float4 lo, float4 hi, const SlotCosts *costs, float (&out)[7]) {
+    if (c & kLeafBit) {
+        const float a = kTriCost * half_area(lo, hi);
+        for (int j = 0; j < 7; ++j) out[j] = a;
+        return;
+    }
+    const float4 a = __ldcg(reinterpret_cast<const float4 *>(&costs[c])), b = __ldcg(reinterpret_cast<const float4 *>(&costs[c]) + 1);
+    out[0] = a.x; out[1] = a.y; out[2] = a.z; out[3] = a.w; out[4] = b.x; out[5] = b.y; out[6] = b.z;
+}
+
+// least L(k) + R(j - k) over k = 1..j-1 (at most 7 slots a side)
+template <int J>
+__device__ __forceinline__ float best_split(const float (&l)[7], const float (&r)[7], uint32_t &k_best) {
+    float best = l[0] + r[J - 2 < 6 ? J - 2 : 6];
+    k_best = 1;
+#pragma unroll
+    for (int k = 2; k < J; ++k) {
+        const float v = l[k - 1] + r[J - k - 1];
+        if (v < best) { best = v; k_best = (uint32_t)k; }
+    }
+    return best;
+}
+
+template <int J>
+__device__ __forceinline__ void cost_of_slots(const float (&l)[7], const float (&r)[7], SlotCosts &s) {
+    uint32_t k;
+    const float v = best_split<J>(l, r, k);
+    // (on a tie the split: subtrees without area still fill their nodes)
+    if (v <= s.c[J - 2]) { s.c[J - 1] = v; s.choice |= k << (4 + 3 * (J - 2)); }
+    else s.c[J - 1] = s.c[J - 2];
+}
+
+__global__ void k_fit(int n, int leaf_max, const uint32_t *__restrict__ vals, const float4 *__restrict__ bmin,
                       const float4 *__restrict__ bmax, const uint32_t *__restrict__ left, const uint32_t *__restrict__ right,
+                      const uint32_t *__restrict__ first, const uint32_t *__restrict__ last,
                       const uint32_t *__restrict__ parent_int, const uint32_t *__restrict__ parent_leaf, uint32_t *counter,
-                      float4 *imin, float4 *imax) {
+                      float4 *imin, float4 *imax, SlotCosts *costs) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= n) return;
     uint32_t node = parent_leaf[j];
     for (int guard = 0; guard < 4096 && node < (uint32_t)(n - 1); ++guard) {
         __threadfence();
         if (atomicAdd(&counter[node], 1u) == 0u) return;   // the other child is not ready yet
+        const uint32_t lc = left[node], rc = right[node];
         float4 l0, l1, r0, r1;
-        child_box(left[node], vals, bmin, bmax, imin, imax, l0, l1);
-        child_box(right[node], vals, bmin, bmax, imin, imax, r0, r1);
-        __stcg(&imin[node], make_float4(fminf(l0.x, r0.x), fminf(l0.y, r0.y), fminf(l0.z, r0.z), 0.0f));
-        __stcg(&imax[node], make_float4(fmaxf(l1.x, r1.x), fmaxf(l1.y, r1.y), fmaxf(l1.z, r1.z), 0.0f));
+        child_box(lc, vals, bmin, bmax, imin, imax, l0, l1);
+        child_box(rc, vals, bmin, bmax, imin, imax, r0, r1);
+        const float4 lo = make_float4(fminf(l0.x, r0.x), fminf(l0.y, r0.y), fminf(l0.z, r0.z), 0.0f);
+        const float4 hi = make_float4(fmaxf(l1.x, r1.x), fmaxf(l1.y, r1.y), fmaxf(l1.z, r1.z), 0.0f);
+        __stcg(&imin[node], lo);
+        __stcg(&imax[node], hi);
+        float l[7], r[7];
+        child_costs(lc, l0, l1, costs, l);
+        child_costs(rc, r0, r1, costs, r);
+        SlotCosts s;
+        const float area = half_area(lo, hi);
+        uint32_t k8;
+        const float as_node = kNodeCost * area + best_split<8>(l, r, k8);
+        const uint32_t tris = last[node] - first[node] + 1u;
+        const float as_leaf = kTriCost * (float)tris * area;
+        const bool leaf = tris <= (uint32_t)leaf_max && as_leaf <= as_node;
+        s.c[0] = leaf ? as_leaf : as_node;
+        s.choice = (leaf ? 1u : 0u) | (k8 << 1);
+        cost_of_slots<2>(l, r, s);
+        cost_of_slots<3>(l, r, s);
+        cost_of_slots<4>(l, r, s);
+        cost_of_slots<5>(l, r, s);
+        cost_of_slots<6>(l, r, s);
+        cost_of_slots<7>(l, r, s);
+        __stcg(reinterpret_cast<float4 *>(&costs[node]), make_float4(s.c[0], s.c[1], s.c[2], s.c[3]));
+        __stcg(reinterpret_cast<float4 *>(&costs[node]) + 1, make_float4(s.c[4], s.c[5], s.c[6], __uint_as_float(s.choice)));
         if (node == 0) return;
         node = parent_int[node];
     }
 }
 
-__device__ __forceinline__ void write_record(float4 *rec, float4 lo, float4 hi, uint32_t a, uint32_t b) {
-    rec[0] = make_float4(lo.x, lo.y, lo.z, __uint_as_float(a));
-    rec[1] = make_float4(hi.x, hi.y, hi.z, __uint_as_float(b));
-}
-
-__device__ __forceinline__ float half_area(float4 lo, float4 hi) {
-    const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
-    return dx * dy + dy * dz + dz * dx;
-}
-
-// --- leaf choice -------------------------------------------------------------------------------
-// A subtree of at most leaf_max triangles becomes one leaf when that is cheaper by the surface-area
-// cost model than keeping its inner nodes.  Per ray that reaches the subtree's box, a leaf costs
-// kTriCost per triangle; an inner node costs kNodeCost plus its two children's costs, each weighted
-// by the share of the node's box area its box has.  The unit is one box test: 2.2 box tests per
-// triangle test and 2 per opened inner node fit the frame times of the 1,000,000-triangle soup at
-// leaves of 1, 2 and 3 triangles, and still do for the 8-wide tree (node cost 1 or triangle cost 4:
-// equal; node cost 4: -11 % on the soup frame, triangle cost 1.2: -6 %; the terrain PathTracer within
-// 0.2 % except node cost 4 and triangle cost 1.2, -3 %).  Scattered small triangles (the soups) end up one per leaf: two
-// boxes cull better than two triangle tests; touching triangles (a heightfield) stay in pairs.
-#ifndef MRT_BVH_TRI_COST
-#define MRT_BVH_TRI_COST 2.2f
-#endif
-#ifndef MRT_BVH_NODE_COST
-#define MRT_BVH_NODE_COST 2.0f
-#endif
-constexpr float kTriCost = MRT_BVH_TRI_COST, kNodeCost = MRT_BVH_NODE_COST;
-constexpr int kLeafCostDepth = 3;   // inner levels of a subtree of up to 4 triangles
-
-struct BinView {
-    const uint32_t *vals;
-    const float4 *bmin, *bmax;
-    const uint32_t *left, *right, *first, *last;
-    const float4 *imin, *imax;
-    __device__ void box(uint32_t c, float4 &lo, float4 &hi) const {
-        if (c & kLeafBit) {
-            const uint32_t t = vals[c & ~kLeafBit];
-            lo = bmin[t];
-            hi = bmax[t];
-        } else {
-            lo = imin[c];
-            hi = imax[c];
-        }
-    }
-    __device__ uint32_t count(uint32_t c) const { return (c & kLeafBit) ? 1u : last[c] - first[c] + 1u; }
-};
-
-template <int D>
-__device__ float subtree_cost(const BinView &v, uint32_t c);
-
-template <int D>
-__device__ float split_cost(const BinView &v, uint32_t c) {
-    float4 lo, hi;
-    v.box(c, lo, hi);
-    const float a = half_area(lo, hi);
-    float cost = kNodeCost;
-    const uint32_t ch[2] = {v.left[c], v.right[c]};
-    for (int k = 0; k < 2; ++k) {
-        float4 l2, h2;
-        v.box(ch[k], l2, h2);
-        const float share = a > 0.0f ? half_area(l2, h2) / a : 1.0f;
-        cost += share * subtree_cost<D - 1>(v, ch[k]);
-    }
-    return cost;
-}
-
-template <int D>
-__device__ float subtree_cost(const BinView &v, uint32_t c) {
-    if (c & kLeafBit) return kTriCost;
-    const float leaf = kTriCost * (float)v.count(c);
-    if constexpr (D == 0) return leaf;
-    else return fminf(leaf, split_cost<D>(v, c));
-}
-
-// inner node c (count <= leaf_max) as one leaf?
-__device__ __forceinline__ bool leaf_by_cost(const BinView &v, uint32_t c) {
-    return kTriCost * (float)v.count(c) <= split_cost<kLeafCostDepth>(v, c);
-}
-
-// one record per child of every internal node (pair at 2 + 2k), plus the root record 0
-__global__ void k_emit(int n, int leaf_max, const uint32_t *__restrict__ vals, const float4 *__restrict__ bmin,
-                       const float4 *__restrict__ bmax, const uint32_t *__restrict__ left, const uint32_t *__restrict__ right,
-                       const uint32_t *__restrict__ first, const uint32_t *__restrict__ last, const float4 *__restrict__ imin,
-                       const float4 *__restrict__ imax, float4 *records) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= n - 1) return;
-    const BinView v{vals, bmin, bmax, left, right, first, last, imin, imax};
-    if (k == 0) {
-        const uint32_t cnt = last[0] - first[0] + 1;
-        if ((int)cnt <= leaf_max && leaf_by_cost(v, 0u)) write_record(records, imin[0], imax[0], first[0], cnt);
-        else write_record(records, imin[0], imax[0], 2u, 0u);
-        write_record(records + 2, make_float4(0, 0, 0, 0), make_float4(0, 0, 0, 0), 0u, 0u);
-    }
-    for (int side = 0; side < 2; ++side) {
-        const uint32_t c = side == 0 ? left[k] : right[k];
-        float4 *rec = records + 2 * (2 + 2 * (size_t)k + side);
-        float4 lo, hi;
-        if (c & kLeafBit) {
-            const uint32_t j = c & ~kLeafBit;
-            lo = bmin[vals[j]];
-            hi = bmax[vals[j]];
-            write_record(rec, lo, hi, j, 1u);
-        } else {
-            lo = imin[c];
-            hi = imax[c];
-            const uint32_t cnt = last[c] - first[c] + 1;
-            if ((int)cnt <= leaf_max && leaf_by_cost(v, c)) write_record(rec, lo, hi, first[c], cnt);
-            else write_record(rec, lo, hi, 2u + 2u * c, 0u);
-        }
-    }
-}
-
-__global__ void k_leaf_tris(uint32_t n, const uint32_t *__restrict__ vals, const float4 *__restrict__ a4,
-                            const float4 *__restrict__ ab4, const float4 *__restrict__ ac4, float4 *out) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= n) return;
-    const uint32_t t = vals[j];
-    const float4 a = a4[t];
-    out[3 * (size_t)j] = make_float4(a.x, a.y, a.z, __uint_as_float(t));
-    out[3 * (size_t)j + 1] = ab4[t];
-    out[3 * (size_t)j + 2] = ac4[t];
-}
-
-__global__ void k_single_leaf(const float4 *bmin, const float4 *bmax, float4 *records) {
-    write_record(records, bmin[0], bmax[0], 0u, 1u);
-}
-
 // ------------------------------ binary -> 8-wide compressed nodes ------------------------------
-// Each wide node starts from the children of one binary internal node (or from the root record) and
-// opens its largest-area internal child until it holds kWide children.  Its box is the union of the
-// children's boxes; per axis the children's planes are quantised on a grid p + 2^E q (16-bit q,
-// lo rounded down and hi up, so every quantised box contains the exact one), the children are
-// placed in slots by the octant of their centre within the node, internal children get consecutive
+// A wide node holds its binary node's two children in 8 slots by the choices above.  Its box is the
+// union of the children's boxes; per axis the children's planes are quantised on a grid p + 2^E q
+// (16-bit q, lo rounded down and hi up, so every quantised box contains the exact one), the children
+// are placed in slots by the octant of their centre within the node, internal children get consecutive
 // node indices (one allocation per node), and the triangles of the leaf children are copied to
-// consecutive records (one allocation per node).  One launch per level of the wide tree.
+// consecutive records (one allocation per node).  One launch per level of the wide tree; a level's size
+// stays on the device (ctrs), so levels follow each other without a host round trip.
 struct CollapseItem {
-    uint32_t rec;     // first seed record: the root record 0 (one seed) or a child pair 2 + 2k (two seeds)
-    uint32_t seeds;   // 1 or 2
+    uint32_t bin;     // binary node (kLeafBit: a single triangle, the whole scene)
     uint32_t node;    // the wide node it becomes
 };
 
-__device__ __forceinline__ bool rec_internal(const float4 *bin, uint32_t r) { return __float_as_int(bin[2 * (size_t)r + 1].w) == 0; }
+struct BinTree {
+    const uint32_t *vals;             // triangle of each place in Morton order
+    const float4 *bmin, *bmax;        // triangle boxes
+    const uint32_t *left, *right, *first, *last;
+    const float4 *imin, *imax;        // inner boxes
+    const SlotCosts *costs;
+    uint32_t n;
+    __device__ bool is_leaf(uint32_t c) const { return (c & kLeafBit) || (costs[c].choice & 1u); }
+};
+
+// ctrs: [0] nodes allocated, [1] error, [2] triangles placed, [kLevelCtr + l] items of level l
+constexpr int kLevelCtr = 4, kMaxLevels = 68;   // the binary tree is at most 62 levels deep
 
 // grid step exponent E of one axis (2^E >= extent / 65534)
 __device__ __forceinline__ int grid_exponent(float lo, float hi) {
@@ -477,45 +476,55 @@ __device__ __forceinline__ uint32_t quantise(float p, double step, float lo, flo
     return (uint32_t)ql | ((uint32_t)qh << 16);
 }
 
-// ctrs[0]: items of the next level, [1]: nodes allocated, [2]: error, [3]: triangles placed
-__global__ void k_collapse(const float4 *__restrict__ bin, uint32_t n_records, const CollapseItem *__restrict__ in,
-                           uint32_t n_in, CollapseItem *out, uint32_t cap, uint4 *nodes, const float4 *__restrict__ mtris,
-                           float4 *tris, uint32_t n_tri, uint32_t *ctrs) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n_in) return;
-    const CollapseItem it = in[i];
-    uint32_t rec[kWide];
-    int m = (int)it.seeds;
-    rec[0] = it.rec;
-    rec[1] = it.rec + 1u;
-    if ((uint64_t)it.rec + (uint64_t)it.seeds > n_records || it.node >= cap) { atomicMax(&ctrs[2], 1u); return; }
-    for (;;) {   // open the internal child with the largest box while there is room
-        if (m >= kWide) break;
-        int best = -1;
-        float best_area = -1.0f;
-        for (int k = 0; k < m; ++k) {
-            if (!rec_internal(bin, rec[k])) continue;
-            const float a = half_area(bin[2 * (size_t)rec[k]], bin[2 * (size_t)rec[k] + 1]);
-            if (a > best_area) { best_area = a; best = k; }
+__device__ void collapse_node(const BinTree &t, CollapseItem it, int level, CollapseItem *out, uint32_t cap, uint4 *nodes,
+                              const float4 *__restrict__ a4, const float4 *__restrict__ ab4,
+                              const float4 *__restrict__ ac4, float4 *tris, uint32_t *ctrs) {
+    const uint32_t n_tri = t.n;
+    if (it.node >= cap) { atomicMax(&ctrs[1], 1u); return; }
+    uint32_t child[kWide];
+    int m = 0;
+    if (t.is_leaf(it.bin)) {   // only the root of a scene of at most kMaxLeafTris triangles
+        child[m++] = it.bin;
+    } else {
+        uint32_t st_node[kWide], st_slots[kWide];
+        int sp = 0;
+        const uint32_t k8 = choice_node_split(t.costs[it.bin].choice);
+        st_node[sp] = t.right[it.bin]; st_slots[sp++] = 8u - k8;
+        st_node[sp] = t.left[it.bin]; st_slots[sp++] = k8;
+        while (sp > 0) {
+            const uint32_t c = st_node[--sp];
+            uint32_t j = min(st_slots[sp], 7u), k = 0;
+            if (!(c & kLeafBit)) {
+                const uint32_t choice = t.costs[c].choice;
+                while (j > 1u && (k = choice_split(choice, j)) == 0u) --j;
+            }
+            if (k == 0u) {   // one slot
+                if (m >= kWide) { atomicMax(&ctrs[1], 1u); return; }
+                child[m++] = c;
+                continue;
+            }
+            if (sp + 2 > kWide) { atomicMax(&ctrs[1], 1u); return; }
+            st_node[sp] = t.right[c]; st_slots[sp++] = j - k;
+            st_node[sp] = t.left[c]; st_slots[sp++] = k;
         }
-        if (best < 0) break;
-        const uint32_t a = __float_as_uint(bin[2 * (size_t)rec[best]].w);
-        if (a < 2u || (uint64_t)a + 1u >= n_records) { atomicMax(&ctrs[2], 1u); return; }
-        rec[best] = a;
-        rec[m++] = a + 1u;
     }
     float4 lo[kWide], hi[kWide];
+    bool internal[kWide];
     float4 nlo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f), nhi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
     for (int k = 0; k < m; ++k) {
-        lo[k] = bin[2 * (size_t)rec[k]];
-        hi[k] = bin[2 * (size_t)rec[k] + 1];
+        const uint32_t c = child[k];
+        if (c & kLeafBit) {
+            const uint32_t tri = t.vals[c & ~kLeafBit];
+            lo[k] = t.bmin[tri];
+            hi[k] = t.bmax[tri];
+        } else {
+            lo[k] = t.imin[c];
+            hi[k] = t.imax[c];
+        }
+        internal[k] = !t.is_leaf(c);
         nlo = make_float4(fminf(nlo.x, lo[k].x), fminf(nlo.y, lo[k].y), fminf(nlo.z, lo[k].z), 0.0f);
         nhi = make_float4(fmaxf(nhi.x, hi[k].x), fmaxf(nhi.y, hi[k].y), fmaxf(nhi.z, hi[k].z), 0.0f);
     }
-    // (keeping the internal children of a full node that hold at most 3 triangles as leaves instead:
-    // 38 % fewer nodes on the 1,000,000-triangle soup, 4.5x the triangle tests, 1.3 % slower)
-    bool internal[kWide];
-    for (int k = 0; k < m; ++k) internal[k] = rec_internal(bin, rec[k]);
     // slots by octant: the child whose centre lies on the high side of axis a prefers slots with bit a set
     const float cx = 0.5f * (nlo.x + nhi.x), cy = 0.5f * (nlo.y + nhi.y), cz = 0.5f * (nlo.z + nhi.z);
     int slot_of[kWide];
@@ -548,17 +557,17 @@ __global__ void k_collapse(const float4 *__restrict__ bin, uint32_t n_records, c
     for (int k = 0; k < m; ++k) {
         child_at[slot_of[k]] = k;
         if (internal[k]) { imask |= 1u << slot_of[k]; ++n_int; }
-        else n_lt += (uint32_t)__float_as_int(hi[k].w);
+        else n_lt += (child[k] & kLeafBit) ? 1u : t.last[child[k]] - t.first[child[k]] + 1u;
     }
-    const uint32_t child_base = n_int ? atomicAdd(&ctrs[1], n_int) : 0u;
-    const uint32_t qpos = n_int ? atomicAdd(&ctrs[0], n_int) : 0u;
-    const uint32_t tri_base = n_lt ? atomicAdd(&ctrs[3], n_lt) : 0u;
+    const uint32_t child_base = n_int ? atomicAdd(&ctrs[0], n_int) : 0u;
+    const uint32_t qpos = n_int ? atomicAdd(&ctrs[kLevelCtr + level + 1], n_int) : 0u;
+    const uint32_t tri_base = n_lt ? atomicAdd(&ctrs[2], n_lt) : 0u;
     if ((uint64_t)child_base + n_int > cap || (uint64_t)qpos + n_int > cap || (uint64_t)tri_base + n_lt > n_tri) {
-        atomicMax(&ctrs[2], 1u);
+        atomicMax(&ctrs[1], 1u);
         return;
     }
     const int ex = grid_exponent(nlo.x, nhi.x), ey = grid_exponent(nlo.y, nhi.y), ez = grid_exponent(nlo.z, nhi.z);
-    if (ex > 127 || ey > 127 || ez > 127) { atomicMax(&ctrs[2], 2u); return; }
+    if (ex > 127 || ey > 127 || ez > 127) { atomicMax(&ctrs[1], 2u); return; }
     const double sx = ldexp(1.0, ex), sy = ldexp(1.0, ey), sz = ldexp(1.0, ez);
     uint32_t w[kNodeWords];
     w[0] = __float_as_uint(nlo.x);
@@ -579,19 +588,37 @@ __global__ void k_collapse(const float4 *__restrict__ bin, uint32_t n_records, c
         w[node_plane_word(1, sl)] = quantise(nlo.y, sy, lo[k].y, hi[k].y);
         w[node_plane_word(2, sl)] = quantise(nlo.z, sz, lo[k].z, hi[k].z);
         if ((imask >> sl) & 1u) {
-            out[qpos + rank] = CollapseItem{__float_as_uint(lo[k].w), 2u, child_base + rank};
+            out[qpos + rank] = CollapseItem{child[k], child_base + rank};
             ++rank;
         } else {
-            const uint32_t first = __float_as_uint(lo[k].w), count = (uint32_t)__float_as_int(hi[k].w);
-            if (count == 0 || count > kMaxLeafTris || (uint64_t)first + count > n_tri) { atomicMax(&ctrs[2], 1u); return; }
+            const uint32_t c = child[k];
+            const uint32_t first = (c & kLeafBit) ? c & ~kLeafBit : t.first[c];
+            const uint32_t count = (c & kLeafBit) ? 1u : t.last[c] - first + 1u;
+            if (count == 0 || count > kMaxLeafTris || (uint64_t)first + count > n_tri) { atomicMax(&ctrs[1], 1u); return; }
             w[kNodeMeta + (sl >> 2)] |= ((((1u << count) - 1u) << 5) | offset) << (8 * (sl & 3));
-            for (uint32_t j = 0; j < count; ++j)
-                for (int c = 0; c < 3; ++c) tris[3 * (size_t)(tri_base + offset + j) + c] = mtris[3 * (size_t)(first + j) + c];
+            for (uint32_t j = 0; j < count; ++j) {
+                const uint32_t tri = t.vals[first + j];
+                const float4 a = a4[tri];
+                float4 *rec = tris + 3 * (size_t)(tri_base + offset + j);
+                rec[0] = make_float4(a.x, a.y, a.z, __uint_as_float(tri));
+                rec[1] = ab4[tri];
+                rec[2] = ac4[tri];
+            }
             offset += count;
         }
     }
     uint4 *dst = nodes + (size_t)it.node * (kNodeWords / 4);
     for (int q = 0; q < kNodeWords / 4; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+}
+
+__global__ void __launch_bounds__(128) k_collapse(BinTree t, const CollapseItem *__restrict__ in, int level, CollapseItem *out,
+                                                  uint32_t cap, uint4 *nodes, const float4 *__restrict__ a4,
+                                                  const float4 *__restrict__ ab4, const float4 *__restrict__ ac4,
+                                                  float4 *tris, uint32_t *ctrs) {
+    if (ctrs[1]) return;   // after an error the level's items may be unwritten
+    const uint32_t n_in = min(ctrs[kLevelCtr + level], cap);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
+        collapse_node(t, in[i], level, out, cap, nodes, a4, ab4, ac4, tris, ctrs);
 }
 
 }  // namespace
@@ -624,108 +651,102 @@ int build_fast_bvh(MrtScene *s) {
         return MRT_ERR_ARG;
     }
     int st = MRT_OK;
-    const uint64_t n_records = 2ull + 2ull * (n > 1 ? n - 1 : 0) + 2ull;
-    st = dev_alloc(ctx, s->fnodes, 32ull * n_records);
-    if (st == MRT_OK) st = dev_alloc(ctx, s->ftris, 48ull * n);
+    st = dev_alloc(ctx, s->ftris, 48ull * n);
     if (st != MRT_OK) return st;
-    DevBuf bmin, bmax, cb, keys[2], vals[2], hist, lft, rgt, fst, lst, pint, pleaf, ctr, imin, imax, mtris;
+    DevBuf bmin, bmax, cb, keys[2], vals[2], hist, total, lft, rgt, fst, lst, pint, pleaf, ctr, imin, imax, costs;
     const uint32_t nblocks = (n + kSortTile - 1) / kSortTile;
     auto A = [&](DevBuf &b, size_t bytes) { if (st == MRT_OK) st = dev_alloc(ctx, b, bytes); };
     A(bmin, 16ull * n); A(bmax, 16ull * n); A(cb, 64);
     A(keys[0], 4ull * n); A(keys[1], 4ull * n); A(vals[0], 4ull * n); A(vals[1], 4ull * n);
-    A(hist, 4ull * 256 * nblocks);
+    A(hist, 4ull * 256 * nblocks); A(total, 4ull * 256);
     A(lft, 4ull * n); A(rgt, 4ull * n); A(fst, 4ull * n); A(lst, 4ull * n);
     A(pint, 4ull * n); A(pleaf, 4ull * n); A(ctr, 4ull * n); A(imin, 16ull * n); A(imax, 16ull * n);
-    A(mtris, 48ull * n);
+    A(costs, sizeof(SlotCosts) * (size_t)n);
     if (st == MRT_OK) {
         const uint32_t init[6] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u, 0u};
         st = cuda_status(ctx, cudaMemcpyAsync(cb.ptr, init, sizeof(init), cudaMemcpyHostToDevice, q), "bvh init");
     }
+    int cur = 0;
     if (st == MRT_OK) {
         const uint32_t g = (n + 255) / 256;
         k_tri_boxes<<<g, 256, 0, q>>>(n, s->dev.tri_a, s->dev.tri_ab, s->dev.tri_ac, (float4 *)bmin.ptr,
                                       (float4 *)bmax.ptr, (uint32_t *)cb.ptr);
         k_morton<<<g, 256, 0, q>>>(n, (const float4 *)bmin.ptr, (const float4 *)bmax.ptr, (const uint32_t *)cb.ptr,
                                    (uint32_t *)keys[0].ptr, (uint32_t *)vals[0].ptr);
-        int cur = 0;
         for (int shift = 0; shift < 30; shift += 8) {
             k_rs_hist<<<nblocks, kSortThreads, 0, q>>>((const uint32_t *)keys[cur].ptr, n, shift, (uint32_t *)hist.ptr, nblocks);
-            k_scan_exclusive<<<1, 1024, 0, q>>>((uint32_t *)hist.ptr, 256u * nblocks);
+            k_rs_scan_rows<<<256, 256, 0, q>>>((uint32_t *)hist.ptr, nblocks, (uint32_t *)total.ptr);
             k_rs_scatter<<<nblocks, kSortThreads, 0, q>>>((const uint32_t *)keys[cur].ptr, (const uint32_t *)vals[cur].ptr,
                                                           (uint32_t *)keys[1 - cur].ptr, (uint32_t *)vals[1 - cur].ptr, n,
-                                                          shift, (const uint32_t *)hist.ptr, nblocks);
+                                                          shift, (const uint32_t *)hist.ptr, nblocks, (const uint32_t *)total.ptr);
             cur = 1 - cur;
         }
-        const uint32_t *skeys = (const uint32_t *)keys[cur].ptr;
-        const uint32_t *svals = (const uint32_t *)vals[cur].ptr;
-        if (n == 1) {
-            k_single_leaf<<<1, 1, 0, q>>>((const float4 *)bmin.ptr, (const float4 *)bmax.ptr, (float4 *)s->fnodes.ptr);
-        } else {
+        if (n > 1) {
+            const uint32_t *svals = (const uint32_t *)vals[cur].ptr;
             cudaMemsetAsync(ctr.ptr, 0, 4ull * n, q);
-            k_karras<<<(n - 1 + 255) / 256, 256, 0, q>>>((int)n, skeys, (uint32_t *)lft.ptr, (uint32_t *)rgt.ptr,
-                                                          (uint32_t *)fst.ptr, (uint32_t *)lst.ptr, (uint32_t *)pint.ptr,
-                                                          (uint32_t *)pleaf.ptr);
-            k_fit<<<(n + 255) / 256, 256, 0, q>>>((int)n, svals, (const float4 *)bmin.ptr, (const float4 *)bmax.ptr,
-                                                  (const uint32_t *)lft.ptr, (const uint32_t *)rgt.ptr,
-                                                  (const uint32_t *)pint.ptr, (const uint32_t *)pleaf.ptr,
-                                                  (uint32_t *)ctr.ptr, (float4 *)imin.ptr, (float4 *)imax.ptr);
-            k_emit<<<(n - 1 + 255) / 256, 256, 0, q>>>((int)n, leaf_max_setting(), svals, (const float4 *)bmin.ptr,
-                                                       (const float4 *)bmax.ptr, (const uint32_t *)lft.ptr,
-                                                       (const uint32_t *)rgt.ptr, (const uint32_t *)fst.ptr,
-                                                       (const uint32_t *)lst.ptr, (const float4 *)imin.ptr,
-                                                       (const float4 *)imax.ptr, (float4 *)s->fnodes.ptr);
+            k_karras<<<(n - 1 + 255) / 256, 256, 0, q>>>((int)n, (const uint32_t *)keys[cur].ptr, (uint32_t *)lft.ptr,
+                                                          (uint32_t *)rgt.ptr, (uint32_t *)fst.ptr, (uint32_t *)lst.ptr,
+                                                          (uint32_t *)pint.ptr, (uint32_t *)pleaf.ptr);
+            k_fit<<<(n + 255) / 256, 256, 0, q>>>((int)n, leaf_max_setting(), svals, (const float4 *)bmin.ptr,
+                                                  (const float4 *)bmax.ptr, (const uint32_t *)lft.ptr,
+                                                  (const uint32_t *)rgt.ptr, (const uint32_t *)fst.ptr,
+                                                  (const uint32_t *)lst.ptr, (const uint32_t *)pint.ptr,
+                                                  (const uint32_t *)pleaf.ptr, (uint32_t *)ctr.ptr, (float4 *)imin.ptr,
+                                                  (float4 *)imax.ptr, (SlotCosts *)costs.ptr);
         }
-        k_leaf_tris<<<(n + 255) / 256, 256, 0, q>>>(n, svals, s->dev.tri_a, s->dev.tri_ab, s->dev.tri_ac,
-                                                    (float4 *)mtris.ptr);
         st = cuda_status(ctx, cudaGetLastError(), "fast bvh kernels");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "fast bvh build");
     }
-    DevBuf *tmp[] = {&bmin, &bmax, &cb, &keys[0], &keys[1], &vals[0], &vals[1], &hist, &lft, &rgt, &fst, &lst,
-                     &pint, &pleaf, &ctr, &imin, &imax};
+    DevBuf *tmp[] = {&cb, &keys[0], &keys[1], &vals[1 - cur], &hist, &total, &pint, &pleaf, &ctr};
     for (DevBuf *b : tmp) dev_free(*b);
-    if (st != MRT_OK) { dev_free(mtris); return st; }
-    // collapse into 8-wide compressed nodes, level by level, from the root record
+    // collapse into 8-wide compressed nodes, level by level, from the root
     DevBuf wide, queue[2], wctr;
-    const uint32_t cap = n;   // wide nodes <= binary internal nodes + 1
+    const uint32_t cap = n;   // every wide node but the root of a single-triangle scene is a binary internal node
     A(wide, 4ull * kNodeWords * cap);
     A(queue[0], sizeof(CollapseItem) * cap);
     A(queue[1], sizeof(CollapseItem) * cap);
-    A(wctr, 16);
-    uint32_t h[4] = {1, 1, 0, 0};   // the root item, the root node
+    uint32_t h[kLevelCtr + kMaxLevels + 1] = {0};
+    A(wctr, sizeof(h));
+    h[0] = 1;              // the root node
+    h[kLevelCtr] = 1;      // the root item
     if (st == MRT_OK) {
-        const CollapseItem root{0u, 1u, 0u};
+        const CollapseItem root{n > 1 ? 0u : kLeafBit, 0u};
         st = cuda_status(ctx, cudaMemcpyAsync(queue[0].ptr, &root, sizeof(root), cudaMemcpyHostToDevice, q), "collapse");
-        if (st == MRT_OK) st = cuda_status(ctx, cudaMemcpyAsync(wctr.ptr, h, 16, cudaMemcpyHostToDevice, q), "collapse");
+        if (st == MRT_OK) st = cuda_status(ctx, cudaMemcpyAsync(wctr.ptr, h, sizeof(h), cudaMemcpyHostToDevice, q), "collapse");
     }
-    int cur_q = 0;
-    for (int level = 0; st == MRT_OK && h[0] > 0 && h[2] == 0; ++level) {
-        if (level > 4096) { st = MRT_ERR_LIMIT; break; }
-        const uint32_t n_in = h[0];
-        cudaMemsetAsync(wctr.ptr, 0, 4, q);
-        k_collapse<<<(n_in + 127) / 128, 128, 0, q>>>((const float4 *)s->fnodes.ptr, (uint32_t)n_records,
-                                                       (const CollapseItem *)queue[cur_q].ptr, n_in,
-                                                       (CollapseItem *)queue[1 - cur_q].ptr, cap, (uint4 *)wide.ptr,
-                                                       (const float4 *)mtris.ptr, (float4 *)s->ftris.ptr, n,
-                                                       (uint32_t *)wctr.ptr);
-        cur_q = 1 - cur_q;
-        st = cuda_status(ctx, cudaMemcpyAsync(h, wctr.ptr, 16, cudaMemcpyDeviceToHost, q), "collapse");
+    const BinTree bt{(const uint32_t *)vals[cur].ptr, (const float4 *)bmin.ptr, (const float4 *)bmax.ptr,
+                     (const uint32_t *)lft.ptr, (const uint32_t *)rgt.ptr, (const uint32_t *)fst.ptr,
+                     (const uint32_t *)lst.ptr, (const float4 *)imin.ptr, (const float4 *)imax.ptr,
+                     (const SlotCosts *)costs.ptr, n};
+    // the first ten levels at once (a million triangles take eight to ten), then four more at a time
+    for (int level = 0; st == MRT_OK && h[1] == 0 && h[kLevelCtr + level] > 0;) {
+        for (const int stop = level + (level == 0 ? 10 : 4); level < stop; ++level) {
+            if (level + 1 > kMaxLevels) { st = MRT_ERR_LIMIT; break; }
+            const uint64_t most = level < 9 ? std::min<uint64_t>(1ull << (3 * level), cap) : cap;   // items of a level
+            const uint32_t blocks = (uint32_t)std::min<uint64_t>((most + 127) / 128, (uint64_t)ctx->sm_count * 16);
+            k_collapse<<<blocks, 128, 0, q>>>(bt, (const CollapseItem *)queue[level & 1].ptr, level,
+                                              (CollapseItem *)queue[1 - (level & 1)].ptr, cap, (uint4 *)wide.ptr,
+                                              s->dev.tri_a, s->dev.tri_ab, s->dev.tri_ac, (float4 *)s->ftris.ptr,
+                                              (uint32_t *)wctr.ptr);
+        }
+        if (st == MRT_OK) st = cuda_status(ctx, cudaGetLastError(), "collapse");
+        if (st == MRT_OK) st = cuda_status(ctx, cudaMemcpyAsync(h, wctr.ptr, sizeof(h), cudaMemcpyDeviceToHost, q), "collapse");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "collapse");
     }
-    if (st == MRT_OK && (h[2] != 0 || h[3] != n)) {
-        set_error(ctx, h[2] == 2 ? "fast bvh: scene extent beyond the 2^127 grid step"
+    if (st == MRT_OK && (h[1] != 0 || h[2] != n)) {
+        set_error(ctx, h[1] == 2 ? "fast bvh: scene extent beyond the 2^127 grid step"
                                  : "fast bvh: inconsistent binary tree while collapsing");
         st = MRT_ERR_LIMIT;
     }
-    const uint64_t n_wide = h[1];
-    if (st == MRT_OK) {   // exact-size copy; the binary records and the scratch go
-        dev_free(s->fnodes);
+    const uint64_t n_wide = h[0];
+    if (st == MRT_OK) {   // exact-size copy; the scratch goes
         st = dev_alloc(ctx, s->fnodes, 4ull * kNodeWords * n_wide);
         if (st == MRT_OK)
             st = cuda_status(ctx, cudaMemcpyAsync(s->fnodes.ptr, wide.ptr, 4ull * kNodeWords * n_wide,
                                                   cudaMemcpyDeviceToDevice, q), "collapse copy");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "collapse copy");
     }
-    DevBuf *tmp2[] = {&wide, &queue[0], &queue[1], &wctr, &mtris};
+    DevBuf *tmp2[] = {&wide, &queue[0], &queue[1], &wctr, &bmin, &bmax, &vals[cur], &lft, &rgt, &fst, &lst, &imin, &imax, &costs};
     for (DevBuf *b : tmp2) dev_free(*b);
     if (st != MRT_OK) return st;
     s->fnode_count = n_wide;
