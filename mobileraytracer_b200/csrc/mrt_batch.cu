@@ -55,15 +55,11 @@ struct BatchState {
     const RenderParams *jobs;   // [max_jobs]
     const DevScene *scenes;     // [max_jobs]
     const WaveDesc *desc;
-    RayRec *rays;
-    NodeRec *nodes;
-    ShadowRec *shadows;
+    WaveRecords rec;
     Level *levels;              // [n_levels + 2]
     float4 *root_rgb;           // [wave]
     uint32_t *root_job;         // [wave] job slot of each camera path
     uint32_t *root_local;       // [wave] path index within its job
-    uint32_t ray_cap;
-    uint32_t shadow_cap;
     int n_levels;
     unsigned long long *counters;   // [0] closest, [1] shadow (real waves); [2], [3] all waves
     uint32_t *work;                 // persistent work counters, 2 per level
@@ -114,7 +110,7 @@ __global__ void k_batch_raygen(BatchState b) {
         rr.parent = 0xFFFFFFFFu;
         rr.slot = 0;
         rr.code = 1u;
-        b.rays[i] = rr;
+        store_ray(b.rec, i, rr);
         b.root_job[i] = sg.job;
         b.root_local[i] = local;
     }
@@ -137,15 +133,13 @@ struct BatchExtendWork {
     __device__ const FastView &view(const BatchLane &lane, const DevScene &) const { return lane.v; }
     __device__ bool begin(uint32_t item, BatchLane &lane, Ray &r) const {
         lane.idx = L.start + item;
-        const RayRec rr = b.rays[lane.idx];
-        lane.job = b.root_job[rr.root];
+        lane.job = b.root_job[b.rec.links[lane.idx].x];
         lane.v = fast_view(b.scenes[lane.job]);
-        r = ray_of(rr);
+        r = load_ray_only(b.rec, lane.idx);
         return true;
     }
     __device__ bool finish(BatchLane &lane, Ray &, bool hit, float t, uint32_t id, const FastTrav &) const {
-        b.nodes[lane.idx].hit_t = t;
-        b.nodes[lane.idx].hit_id = hit ? id : MRT_HIT_NONE;
+        store_hit(b.rec, lane.idx, hit, t, id);
         return false;
     }
 };
@@ -159,22 +153,14 @@ struct BatchShadowWork {
     __device__ const DevScene &scene(const BatchLane &lane, const DevScene &) const { return b.scenes[lane.job]; }
     __device__ const FastView &view(const BatchLane &lane, const DevScene &) const { return lane.v; }
     __device__ bool begin(uint32_t item, BatchLane &lane, Ray &r, float &dist) const {
-        const ShadowRec sr = b.shadows[item];
         lane.idx = item;
-        lane.job = b.root_job[b.rays[sr.node].root];
+        lane.job = b.root_job[b.rec.links[b.rec.shadow_to[item].x].x];
         lane.v = fast_view(b.scenes[lane.job]);
-        r.o = V3{sr.ox, sr.oy, sr.oz};
-        r.d = V3{sr.dx, sr.dy, sr.dz};
-        r.depth = 0;
-        r.exclude = sr.exclude;
-        dist = sr.dist;
+        r = load_shadow(b.rec, item, dist);
         return true;
     }
     __device__ void finish(BatchLane &lane, bool occluded) const {
-        if (occluded) {
-            const ShadowRec &sr = b.shadows[lane.idx];
-            atomicOr(&b.nodes[sr.node].occluded, 1u << (sr.j & 31u));
-        }
+        if (occluded) mark_occluded(b.rec, lane.idx);
     }
 };
 
@@ -243,8 +229,8 @@ constexpr int kBatchThreadsPerSm = MRT_BATCH_THREADS_PER_SM;
 template <int kBlock, int Q>
 __global__ void __launch_bounds__(kBlock, kBatchThreadsPerSm / kBlock) k_batch_extend(BatchState b, int level) {
     Level L = b.levels[level];
-    L.start = min(L.start, b.ray_cap);
-    L.count = min(L.count, b.ray_cap - L.start);
+    L.start = min(L.start, b.rec.ray_cap);
+    L.count = min(L.count, b.rec.ray_cap - L.start);
     BatchExtendWork work{b, L, b.work + 2 * level};
     BatchLane lane;
     persistent_closest<false, Q>(b.scenes[0], work, lane);
@@ -256,7 +242,7 @@ __global__ void __launch_bounds__(kBlock, kBatchThreadsPerSm / kBlock) k_batch_e
 
 template <int kBlock>
 __global__ void __launch_bounds__(kBlock, kBatchThreadsPerSm / kBlock) k_batch_shadow(BatchState b, int level) {
-    const uint32_t n = min(b.levels[level].shadow_count, b.shadow_cap);
+    const uint32_t n = min(b.levels[level].shadow_count, b.rec.shadow_cap);
     BatchShadowWork work{b, n, b.work + 2 * level + 1};
     BatchLane lane;
     persistent_any(b.scenes[0], work, lane);
@@ -287,14 +273,14 @@ __device__ __forceinline__ void shade_direct_node(const DevScene &s, const Rende
     const Ray r = ray_of(rr);
     Isect it;
     if (!make_isect(s, r, hit_id, it)) return;
-    nd.flags = kEmit;   // resolves to the value in `point`
-    nd.point = shade_direct(s, p, st, r, it);
+    nd.flags = kEmit;   // resolves to the value in `kd`
+    nd.kd = shade_direct(s, p, st, r, it);
 }
 
 __global__ void __launch_bounds__(128) k_batch_shade(BatchState b, int level) {
     Level L = b.levels[level];
-    L.start = min(L.start, b.ray_cap);
-    L.count = min(L.count, b.ray_cap - L.start);
+    L.start = min(L.start, b.rec.ray_cap);
+    L.count = min(L.count, b.rec.ray_cap - L.start);
     Level *next = &b.levels[level + 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) next->start = L.start + L.count;
     const uint32_t next_start = L.start + L.count;
@@ -312,38 +298,40 @@ __global__ void __launch_bounds__(128) k_batch_shade(BatchState b, int level) {
         Stream st;
         uint32_t job = 0;
         if (active) {
-            rr = b.rays[idx];
+            rr = load_ray(b.rec, idx);
+            const uint2 hit = b.rec.hits[idx];
             job = b.root_job[rr.root];
             const RenderParams &p = b.jobs[job];
             const DevScene &s = b.scenes[job];
             st = stream_of(p, b.root_local[rr.root]);
-            const NodeRec &in = b.nodes[idx];
-            if (direct_shader(p.shader)) shade_direct_node(s, p, rr, in.hit_id, in.hit_t, st, o);
-            else shade_ray(s, p, rr, in.hit_id, in.hit_t, st, o);
-            store_node(b.nodes[idx], o.nd);
+            if (direct_shader(p.shader)) shade_direct_node(s, p, rr, hit.y, bitsf(hit.x), st, o);
+            else shade_ray(s, p, rr, hit.y, bitsf(hit.x), st, o);
+            store_node(b.rec, idx, o.nd);
         }
         const uint32_t cbase = warp_alloc(o.n_child, &next->count);
         const uint32_t sbase = warp_alloc(o.n_shadow, &b.levels[level].shadow_count);
         if (!active) continue;
         const DevScene &s = b.scenes[job];
-        emit_children(s, o, rr, st, idx, next_start + cbase, b.rays, b.ray_cap);
-        emit_shadows(s, b.jobs[job], st, o, rr, idx, sbase, b.shadows, b.shadow_cap);
+        emit_children(s, o, rr, st, idx, next_start + cbase, b.rec);
+        emit_shadows(s, b.jobs[job], st, o, rr, idx, sbase, b.rec);
     }
 }
 
 __global__ void __launch_bounds__(128) k_batch_resolve(BatchState b, int level) {
     Level L = b.levels[level];
-    L.start = min(L.start, b.ray_cap);
-    L.count = min(L.count, b.ray_cap - L.start);
+    L.start = min(L.start, b.rec.ray_cap);
+    L.count = min(L.count, b.rec.ray_cap - L.start);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < L.count; i += gridDim.x * blockDim.x) {
         const uint32_t idx = L.start + i;
-        const NodeRec &nd = b.nodes[idx];
-        const RayRec &rr = b.rays[idx];
+        NodeRec nd;
+        RayRec rr;
+        load_node(b.rec, idx, nd);
+        load_links(b.rec, idx, rr);
         V3 rgb{0.0f, 0.0f, 0.0f};
         bool flag = false;
         const uint32_t kind = nd.flags & 3u;
         if (kind == kEmit) {
-            rgb = nd.point;
+            rgb = nd.kd;
             flag = true;
         } else if (kind == kShaded) {   // misses and cut nodes are black
             const uint32_t job = b.root_job[rr.root];
@@ -354,9 +342,7 @@ __global__ void __launch_bounds__(128) k_batch_resolve(BatchState b, int level) 
         if (rr.parent == 0xFFFFFFFFu) {
             b.root_rgb[rr.root] = make_float4(rgb.x, rgb.y, rgb.z, flag ? 1.0f : 0.0f);
         } else {
-            NodeRec &pn = b.nodes[rr.parent];
-            pn.child[rr.slot] = rgb;
-            if (flag) atomicOr(&pn.child_flag, 1u << rr.slot);
+            store_child(b.rec, rr.parent, rr.slot, rgb, flag);
         }
     }
 }
@@ -456,16 +442,14 @@ BatchState state_of(MrtBatch *b, int pipe) {
     s.jobs = (const RenderParams *)b->d_jobs.ptr;
     s.scenes = (const DevScene *)b->d_scenes.ptr;
     s.desc = (const WaveDesc *)P.d_desc.ptr;
-    s.rays = (RayRec *)P.d_rays.ptr;
-    s.nodes = (NodeRec *)P.d_nodes.ptr;
-    s.shadows = (ShadowRec *)P.d_shadows.ptr;
     s.levels = (Level *)P.d_levels.ptr;
     s.root_rgb = (float4 *)P.d_root_rgb.ptr;
     s.root_job = (uint32_t *)P.d_root_job.ptr;
     s.root_local = (uint32_t *)P.d_root_local.ptr;
-    s.ray_cap = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)b->wave_cap * (b->n_levels + 2));
-    s.shadow_cap = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)b->wave_cap *
-                                                                   std::max(1u, b->opts.max_spl) * 2ull);
+    const uint32_t ray_cap = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)b->wave_cap * (b->n_levels + 2));
+    const uint32_t shadow_cap = (uint32_t)std::min<uint64_t>(0xFFFFFFF0ull, (uint64_t)b->wave_cap *
+                                                                          std::max(1u, b->opts.max_spl) * 2ull);
+    s.rec = wave_records(P.d_rays.ptr, P.d_nodes.ptr, P.d_shadows.ptr, ray_cap, shadow_cap);
     s.n_levels = b->n_levels;
     s.counters = (unsigned long long *)b->d_counters.ptr;
     s.work = (uint32_t *)P.d_work.ptr;
@@ -858,9 +842,9 @@ int mrt_batch_create(MrtContext *ctx, const MrtBatchOpts *opts, MrtBatch **out) 
         BatchPipe &P = b->pipes[p];
         st = cuda_status(ctx, cudaStreamCreateWithFlags(&P.stream, cudaStreamNonBlocking), "cudaStreamCreate");
         A(P.d_desc, sizeof(WaveDesc));
-        A(P.d_rays, sizeof(RayRec) * ray_cap);
-        A(P.d_nodes, sizeof(NodeRec) * ray_cap);
-        A(P.d_shadows, sizeof(ShadowRec) * shadow_cap);
+        A(P.d_rays, kRayBytes * ray_cap);
+        A(P.d_nodes, kNodeBytes * ray_cap);
+        A(P.d_shadows, kShadowBytes * shadow_cap);
         A(P.d_levels, sizeof(Level) * (b->n_levels + 2));
         A(P.d_root_rgb, sizeof(float4) * b->wave_cap);
         A(P.d_root_job, sizeof(uint32_t) * b->wave_cap);

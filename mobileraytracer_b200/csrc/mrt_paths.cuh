@@ -88,11 +88,11 @@ __device__ __forceinline__ void path_shade(const DevScene &s, const RenderParams
         nd.child_flag = 0;
         nd.hit_id = hit_id;
         nd.hit_t = hit_t;
-        nd.point = V3{0, 0, 0};
+        nd.kd = V3{0, 0, 0};
         Isect it;
         if (hit_id != MRT_HIT_NONE && make_isect(s, r, hit_id, it)) {
             nd.flags = kEmit;
-            nd.point = shade_direct(s, p, L.st, r, it);
+            nd.kd = shade_direct(s, p, L.st, r, it);
         }
     } else {
         shade_ray(s, p, rr, hit_id, hit_t, L.st, o);

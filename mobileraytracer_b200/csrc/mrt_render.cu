@@ -269,7 +269,7 @@ __global__ void k_wave_raygen(RenderParams p, WaveState w) {
         rr.parent = 0xFFFFFFFFu;
         rr.slot = 0;
         rr.code = 1u;
-        w.rays[i] = rr;
+        store_ray(w.rec, i, rr);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         w.levels[0].start = 0;
@@ -282,12 +282,11 @@ __global__ void __launch_bounds__(128) k_wave_extend(DevScene s, WaveState w, in
     const Level L = clamp_level(w, w.levels[level]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < L.count; i += gridDim.x * blockDim.x) {
         const uint32_t idx = L.start + i;
-        const Ray r = ray_of(w.rays[idx]);
+        const Ray r = load_ray_only(w.rec, idx);
         float len;
         uint32_t id;
         const bool hit = scene_closest<ACCEL, MODE>(s, r, len, id);
-        w.nodes[idx].hit_t = len;
-        w.nodes[idx].hit_id = hit ? id : MRT_HIT_NONE;
+        store_hit(w.rec, idx, hit, len, id);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[0], (unsigned long long)L.count);
 }
@@ -304,23 +303,25 @@ __device__ __forceinline__ void shade_slot(const DevScene &s, const RenderParams
     RayRec rr;
     Stream st;
     if (active) {
-        rr = w.rays[idx];
+        rr = load_ray(w.rec, idx);
+        const uint2 hit = w.rec.hits[idx];
         Task k;
         uint32_t pixel, sample;
         root_task(p, w, rr.root, k, pixel, sample);
         st = make_stream(p.seed, pixel, sample, p.strata, p.constant_value);
-        shade_ray(s, p, rr, w.nodes[idx].hit_id, w.nodes[idx].hit_t, st, o);
-        store_node(w.nodes[idx], o.nd);
+        shade_ray(s, p, rr, hit.y, bitsf(hit.x), st, o);
+        store_node(w.rec, idx, o.nd);
     }
     // queue compaction: one atomic per warp for children, one for shadow rays
     const uint32_t cbase = warp_alloc(o.n_child, &next->count);
     const uint32_t sbase = warp_alloc(o.n_shadow, &w.levels[level].shadow_count);
     if (!active) return;
-    emit_children(s, o, rr, st, idx, next_start + cbase, w.rays, w.ray_cap);
-    emit_shadows(s, p, st, o, rr, idx, sbase, w.shadows, w.shadow_cap);
+    emit_children(s, o, rr, st, idx, next_start + cbase, w.rec);
+    emit_shadows(s, p, st, o, rr, idx, sbase, w.rec);
 }
 
-__global__ void __launch_bounds__(128) k_wave_shade(DevScene s, RenderParams p, WaveState w, int level) {
+// (8 blocks per SM: glass room 2.13 ms a frame against 2.18 at 7 and 2.19 at 5)
+__global__ void __launch_bounds__(128, 8) k_wave_shade(DevScene s, RenderParams p, WaveState w, int level) {
     const Level L = clamp_level(w, w.levels[level]);
     Level *next = &w.levels[level + 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) next->start = L.start + L.count;
@@ -367,7 +368,7 @@ __global__ void __launch_bounds__(128) k_wave_shade_sorted(DevScene s, RenderPar
         for (int r = 0; r < kSortRounds; ++r) {
             const uint32_t j = r * 128u + threadIdx.x;
             const uint32_t idx = L.start + base + j;
-            const uint32_t c = j < n_here ? shade_class(s, p, w.rays[idx], w.nodes[idx].hit_id) : 3u;
+            const uint32_t c = j < n_here ? shade_class(s, p, load_ray_only(w.rec, idx).depth, w.rec.hits[idx].y) : 3u;
             classes |= c << (2 * r);
 #pragma unroll
             for (uint32_t k = 0; k < (uint32_t)kShadeClasses; ++k) {
@@ -403,15 +404,11 @@ __global__ void __launch_bounds__(128) k_wave_shade_sorted(DevScene s, RenderPar
 
 template <int ACCEL, int MODE>
 __global__ void __launch_bounds__(128) k_wave_shadow(DevScene s, WaveState w, int level) {
-    const uint32_t n = min(w.levels[level].shadow_count, w.shadow_cap);
+    const uint32_t n = min(w.levels[level].shadow_count, w.rec.shadow_cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const ShadowRec sr = w.shadows[i];
-        Ray r;
-        r.o = V3{sr.ox, sr.oy, sr.oz};
-        r.d = V3{sr.dx, sr.dy, sr.dz};
-        r.depth = 0;
-        r.exclude = sr.exclude;
-        if (scene_occ<ACCEL, MODE>(s, r, sr.dist)) atomicOr(&w.nodes[sr.node].occluded, 1u << (sr.j & 31u));
+        float dist;
+        const Ray r = load_shadow(w.rec, i, dist);
+        if (scene_occ<ACCEL, MODE>(s, r, dist)) mark_occluded(w.rec, i);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[1], (unsigned long long)n);
 }
@@ -432,12 +429,11 @@ struct ExtendWork {
     __device__ const DevScene &view(const L &, const DevScene &s) const { return s; }
     __device__ bool begin(uint32_t item, WaveLane &lane, Ray &r) const {
         lane.idx = L.start + item;
-        r = ray_of(w.rays[lane.idx]);
+        r = load_ray_only(w.rec, lane.idx);
         return true;
     }
     __device__ bool finish(WaveLane &lane, Ray &, bool hit, float t, uint32_t id, const FastTrav &) const {
-        w.nodes[lane.idx].hit_t = t;
-        w.nodes[lane.idx].hit_id = hit ? id : MRT_HIT_NONE;
+        store_hit(w.rec, lane.idx, hit, t, id);
         return false;
     }
 };
@@ -452,20 +448,12 @@ struct ShadowWork {
     template <class L>
     __device__ const DevScene &view(const L &, const DevScene &s) const { return s; }
     __device__ bool begin(uint32_t item, WaveLane &lane, Ray &r, float &dist) const {
-        const ShadowRec sr = w.shadows[item];
         lane.idx = item;
-        r.o = V3{sr.ox, sr.oy, sr.oz};
-        r.d = V3{sr.dx, sr.dy, sr.dz};
-        r.depth = 0;
-        r.exclude = sr.exclude;
-        dist = sr.dist;
+        r = load_shadow(w.rec, item, dist);
         return true;
     }
     __device__ void finish(WaveLane &lane, bool occluded) const {
-        if (occluded) {
-            const ShadowRec &sr = w.shadows[lane.idx];
-            atomicOr(&w.nodes[sr.node].occluded, 1u << (sr.j & 31u));
-        }
+        if (occluded) mark_occluded(w.rec, lane.idx);
     }
 };
 
@@ -494,7 +482,7 @@ __global__ void __launch_bounds__(128, kGridBlocksPerSm) k_wave_extend_grid(DevS
 }
 
 __global__ void __launch_bounds__(128, kWaveBlocksPerSm) k_wave_shadow_fast(DevScene s, WaveState w, int level, uint32_t *ctr) {
-    const uint32_t n = min(w.levels[level].shadow_count, w.shadow_cap);
+    const uint32_t n = min(w.levels[level].shadow_count, w.rec.shadow_cap);
     ShadowWork work{w, n, ctr};
     WaveLane lane;
     persistent_any(s, work, lane);
@@ -546,13 +534,15 @@ __global__ void __launch_bounds__(128) k_wave_resolve(DevScene s, RenderParams p
     const Level L = clamp_level(w, w.levels[level]);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < L.count; i += gridDim.x * blockDim.x) {
         const uint32_t idx = L.start + i;
-        const NodeRec &nd = w.nodes[idx];
-        const RayRec &rr = w.rays[idx];
+        NodeRec nd;
+        RayRec rr;
+        load_node(w.rec, idx, nd);
+        load_links(w.rec, idx, rr);
         V3 rgb{0.0f, 0.0f, 0.0f};
         bool flag = false;
         const uint32_t kind = nd.flags & 3u;
         if (kind == kEmit) {
-            rgb = nd.point;
+            rgb = nd.kd;
             flag = true;
         } else if (kind == kShaded) {   // misses and cut nodes are black
             Task k;
@@ -564,9 +554,7 @@ __global__ void __launch_bounds__(128) k_wave_resolve(DevScene s, RenderParams p
         if (rr.parent == 0xFFFFFFFFu) {
             w.root_rgb[rr.root] = make_float4(rgb.x, rgb.y, rgb.z, flag ? 1.0f : 0.0f);
         } else {
-            NodeRec &pn = w.nodes[rr.parent];
-            pn.child[rr.slot] = rgb;
-            if (flag) atomicOr(&pn.child_flag, 1u << rr.slot);
+            store_child(w.rec, rr.parent, rr.slot, rgb, flag);
         }
     }
 }
@@ -922,23 +910,19 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         if (ray_cap > 0xFFFFFFF0ull) { set_error(ctx, "mrt_render: wave too large"); return MRT_ERR_ARG; }
         if (2 * (levels + 1) > 64) { set_error(ctx, "mrt_render: depth_max above 30"); return MRT_ERR_ARG; }
         if (!paths) {   // the wavefront's queues (whole-path launches keep their state per lane)
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[1], sizeof(RayRec) * ray_cap);
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], sizeof(NodeRec) * ray_cap);
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], sizeof(ShadowRec) * shadow_cap);
+            if (st == MRT_OK) st = ensure(ctx, ctx->wave[1], kRayBytes * ray_cap);
+            if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], kNodeBytes * ray_cap);
+            if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], kShadowBytes * shadow_cap);
         }
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[4], sizeof(Level) * (levels + 2));
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[5], sizeof(float4) * wave);
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[6], 16);
         if (st != MRT_OK) return st;
         WaveState w{};
-        w.rays = (RayRec *)ctx->wave[1].ptr;
-        w.nodes = (NodeRec *)ctx->wave[2].ptr;
-        w.shadows = (ShadowRec *)ctx->wave[3].ptr;
+        w.rec = wave_records(ctx->wave[1].ptr, ctx->wave[2].ptr, ctx->wave[3].ptr, (uint32_t)ray_cap, (uint32_t)shadow_cap);
         w.levels = (Level *)ctx->wave[4].ptr;
         w.root_rgb = (float4 *)ctx->wave[5].ptr;
         w.counters = (unsigned long long *)ctx->wave[6].ptr;
-        w.ray_cap = (uint32_t)ray_cap;
-        w.shadow_cap = (uint32_t)shadow_cap;
         // per-material shade queues where the scene mixes diffuse with mirror / glass materials
         w.sort_shading = (o->flags & MRT_RENDER_SHADE_QUEUES) && s->mixed_materials ? 1u : 0u;
         cudaMemsetAsync(w.counters, 0, 16, q);
@@ -1142,11 +1126,12 @@ constexpr size_t kNaLevels = 512;                                   // Level x (
 constexpr size_t kNaRoot = 1024;                                    // float4 x wave
 constexpr size_t kNaRays = kNaRoot + 16ull * kNoAllocWave;
 constexpr size_t kNaRayCap = (size_t)kNoAllocWave * (kNoAllocLevels + 2);
-constexpr size_t kNaNodes = kNaRays + sizeof(RayRec) * kNaRayCap;
-constexpr size_t kNaShadows = kNaNodes + sizeof(NodeRec) * kNaRayCap;
+constexpr size_t kNaNodes = kNaRays + kRayBytes * kNaRayCap;
+constexpr size_t kNaShadows = kNaNodes + kNodeBytes * kNaRayCap;
 constexpr size_t kNaShadowCap = (size_t)kNoAllocWave * kNoAllocMaxSpl * 2;
-constexpr size_t kNoAllocScratchBytes = (kNaShadows + sizeof(ShadowRec) * kNaShadowCap + 255) & ~(size_t)255;
+constexpr size_t kNoAllocScratchBytes = (kNaShadows + kShadowBytes * kNaShadowCap + 255) & ~(size_t)255;
 static_assert(sizeof(Level) * (kNoAllocLevels + 2) <= kNaRoot - kNaLevels, "level table overlaps");
+static_assert(kNaRays % 32 == 0 && kNaNodes % 32 == 0 && kNaShadows % 32 == 0, "records are moved 32 bytes at a time");
 static_assert(kNoAllocScratchBytes <= 12u * 1024u * 1024u, "scratch above 12 MiB");
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
@@ -1239,14 +1224,12 @@ extern "C" int mrt_render_noalloc(MrtScene *s, const MrtCamera *cam, const MrtRe
     } else {
         const int levels = std::max(1, o->depth_max + 1);
         WaveState w{};
-        w.rays = reinterpret_cast<RayRec *>(scratch + kNaRays);
-        w.nodes = reinterpret_cast<NodeRec *>(scratch + kNaNodes);
-        w.shadows = reinterpret_cast<ShadowRec *>(scratch + kNaShadows);
+        w.rec = wave_records(scratch + kNaRays, scratch + kNaNodes, scratch + kNaShadows,
+                             (uint32_t)std::min<size_t>(kNaRayCap, (size_t)kNoAllocWave * (levels + 2)),
+                             (uint32_t)std::min<size_t>(kNaShadowCap, (size_t)kNoAllocWave * o->spl * 2));
         w.levels = reinterpret_cast<Level *>(scratch + kNaLevels);
         w.root_rgb = reinterpret_cast<float4 *>(scratch + kNaRoot);
         w.counters = reinterpret_cast<unsigned long long *>(scratch + kNaWaveCounters);
-        w.ray_cap = (uint32_t)std::min<size_t>(kNaRayCap, (size_t)kNoAllocWave * (levels + 2));
-        w.shadow_cap = (uint32_t)std::min<size_t>(kNaShadowCap, (size_t)kNoAllocWave * o->spl * 2);
         cudaMemsetAsync(w.counters, 0, 16, q);
         const uint64_t total_roots = (uint64_t)p.n_tasks * o->spp;
         p.task_base = 0;

@@ -138,7 +138,7 @@ __device__ __forceinline__ V3 shade_direct(const DevScene &s, const RenderParams
 enum NodeKind : uint32_t { kMiss = 0, kEmit = 1, kCut = 2, kShaded = 3 };
 enum NodeFlag : uint32_t { kHasIndirect = 4, kRRScaled = 8, kKdPos = 16, kKsPos = 32, kKtPos = 64 };
 
-struct RayRec {          // 48 bytes
+struct RayRec {
     float ox, oy, oz, dx, dy, dz;
     int32_t depth;
     uint32_t exclude;
@@ -148,24 +148,137 @@ struct RayRec {          // 48 bytes
     uint32_t code;       // path-tree code keying the stream (root 1, child code*4 + slot + 1)
 };
 
-struct NodeRec {         // 128 bytes
+struct NodeRec {
     uint32_t flags;      // kind | NodeFlag
     uint32_t occluded;   // bit j: shadow ray of light sample j was blocked
     float hit_t;
     uint32_t hit_id;
-    V3 kd, ks, kt;       // 36
-    V3 point, normal;    // 24 (or rgb of an emitter in `point`)
-    V3 child[3];         // 36
+    V3 kd, ks, kt;       // (kd: the radiance of an emitter)
+    V3 point, normal;
+    V3 child[3];
     uint32_t child_flag; // bit s: child s reported a light hit
-    uint32_t pad[3];
 };
 
-struct ShadowRec {       // 40 bytes
+struct ShadowRec {
     float ox, oy, oz, dx, dy, dz, dist;
     uint32_t node;
     uint32_t j;
     uint32_t exclude;
 };
+
+// The records in memory.  What one kernel reads of a record is one aligned piece of 8, 16 or 32 bytes
+// moved by one instruction, so a warp's 32 records fill the sectors they touch:
+//   rays       32 B   origin, direction, depth, exclude        (extend, shade)
+//   links      16 B   root, parent, slot, code                 (shade, resolve)
+//   hits        8 B   distance bits, hit id                    (extend -> shade)
+//   nodes     128 B   four 32-B pieces: flags, occluded, kd, kt.y, kt.z | point, normal, ks.x, ks.y |
+//                     ks.z, kt.x, -, -, child 2 | child 0, child 1; a child is rgb and its light flag.
+//                     A miss, a cut node and an emitter (radiance in kd) use the first piece only, a
+//                     diffuse node the first two and child 0.
+//   shadows    32 B   origin, direction, distance, exclude     (shadow)
+//   shadow_to   8 B   node, light sample                       (shadow, where occluded)
+// As 48-, 128- and 40-byte structures of 4-byte members every member's store touched 32 sectors a warp:
+// 49 M store sectors in the first shade launch of the 512x512x4 glass room PathTracer, the mean launch
+// 157 us (90 us now) and the mean resolve launch 68 us (38 us), the frame 3.36 ms (2.19 ms); the
+// 1024x1024x16 terrain PathTracer 35.3 ms (31.6 ms).
+constexpr size_t kRayBytes = 48, kNodeBytes = 136, kShadowBytes = 40;
+struct WaveRecords {
+    uint4 *rays;         // 2 per ray
+    uint4 *links;
+    uint2 *hits;
+    uint4 *nodes;        // 8 per node
+    uint4 *shadows;      // 2 per shadow ray
+    uint2 *shadow_to;
+    uint32_t ray_cap;
+    uint32_t shadow_cap;
+};
+
+// the pieces carved from three buffers of kRayBytes, kNodeBytes (x ray_cap) and kShadowBytes (x shadow_cap)
+inline WaveRecords wave_records(void *rays, void *nodes, void *shadows, uint32_t ray_cap, uint32_t shadow_cap) {
+    WaveRecords w;
+    w.rays = static_cast<uint4 *>(rays);
+    w.links = w.rays + 2 * (size_t)ray_cap;
+    w.nodes = static_cast<uint4 *>(nodes);
+    w.hits = reinterpret_cast<uint2 *>(w.nodes + 8 * (size_t)ray_cap);
+    w.shadows = static_cast<uint4 *>(shadows);
+    w.shadow_to = reinterpret_cast<uint2 *>(w.shadows + 2 * (size_t)shadow_cap);
+    w.ray_cap = ray_cap;
+    w.shadow_cap = shadow_cap;
+    return w;
+}
+
+// 32 bytes at a 32-byte-aligned address in one instruction (sm_100).  No kernel stores to a record that
+// it also loads, so a load may move past stores.
+__device__ __forceinline__ void load_32b(const uint4 *p, uint4 &a, uint4 &b) {
+    asm("ld.global.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w)
+                 : "l"(p));
+}
+__device__ __forceinline__ void store_32b(uint4 *p, const uint4 &a, const uint4 &b) {
+    asm volatile("st.global.v8.u32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+                 :: "l"(p), "r"(a.x), "r"(a.y), "r"(a.z), "r"(a.w), "r"(b.x), "r"(b.y), "r"(b.z), "r"(b.w)
+                 : "memory");
+}
+__device__ __forceinline__ uint32_t fbits(float f) { return __float_as_uint(f); }
+__device__ __forceinline__ float bitsf(uint32_t u) { return __uint_as_float(u); }
+
+__device__ __forceinline__ void store_ray(const WaveRecords &w, uint32_t i, const RayRec &r) {
+    store_32b(w.rays + 2 * (size_t)i, make_uint4(fbits(r.ox), fbits(r.oy), fbits(r.oz), fbits(r.dx)),
+              make_uint4(fbits(r.dy), fbits(r.dz), (uint32_t)r.depth, r.exclude));
+    w.links[i] = make_uint4(r.root, r.parent, r.slot, r.code);
+}
+__device__ __forceinline__ Ray load_ray_only(const WaveRecords &w, uint32_t i) {
+    uint4 a, b;
+    load_32b(w.rays + 2 * (size_t)i, a, b);
+    Ray r;
+    r.o = V3{bitsf(a.x), bitsf(a.y), bitsf(a.z)};
+    r.d = V3{bitsf(a.w), bitsf(b.x), bitsf(b.y)};
+    r.depth = (int32_t)b.z;
+    r.exclude = b.w;
+    return r;
+}
+__device__ __forceinline__ void load_links(const WaveRecords &w, uint32_t i, RayRec &r) {
+    const uint4 l = w.links[i];
+    r.root = l.x;
+    r.parent = l.y;
+    r.slot = l.z;
+    r.code = l.w;
+}
+__device__ __forceinline__ RayRec load_ray(const WaveRecords &w, uint32_t i) {
+    const Ray q = load_ray_only(w, i);
+    RayRec r;
+    r.ox = q.o.x; r.oy = q.o.y; r.oz = q.o.z;
+    r.dx = q.d.x; r.dy = q.d.y; r.dz = q.d.z;
+    r.depth = q.depth;
+    r.exclude = q.exclude;
+    load_links(w, i, r);
+    return r;
+}
+
+__device__ __forceinline__ void store_shadow(const WaveRecords &w, uint32_t i, const ShadowRec &s) {
+    store_32b(w.shadows + 2 * (size_t)i, make_uint4(fbits(s.ox), fbits(s.oy), fbits(s.oz), fbits(s.dx)),
+              make_uint4(fbits(s.dy), fbits(s.dz), fbits(s.dist), s.exclude));
+    w.shadow_to[i] = make_uint2(s.node, s.j);
+}
+__device__ __forceinline__ Ray load_shadow(const WaveRecords &w, uint32_t i, float &dist) {
+    uint4 a, b;
+    load_32b(w.shadows + 2 * (size_t)i, a, b);
+    Ray r;
+    r.o = V3{bitsf(a.x), bitsf(a.y), bitsf(a.z)};
+    r.d = V3{bitsf(a.w), bitsf(b.x), bitsf(b.y)};
+    r.depth = 0;
+    dist = bitsf(b.z);
+    r.exclude = b.w;
+    return r;
+}
+// light sample j of the node of shadow ray i is blocked
+__device__ __forceinline__ void mark_occluded(const WaveRecords &w, uint32_t i) {
+    const uint2 to = w.shadow_to[i];
+    atomicOr(reinterpret_cast<uint32_t *>(w.nodes + 8 * (size_t)to.x) + 1, 1u << (to.y & 31u));
+}
+__device__ __forceinline__ void store_hit(const WaveRecords &w, uint32_t i, bool hit, float t, uint32_t id) {
+    w.hits[i] = make_uint2(fbits(t), hit ? id : MRT_HIT_NONE);
+}
 
 struct Level {
     uint32_t start;
@@ -175,13 +288,9 @@ struct Level {
 };
 
 struct WaveState {
-    RayRec *rays;
-    NodeRec *nodes;
-    ShadowRec *shadows;
+    WaveRecords rec;
     Level *levels;           // [max_levels + 1]
     float4 *root_rgb;        // per wave root: rgb, flag
-    uint32_t ray_cap;
-    uint32_t shadow_cap;
     uint32_t root_first;     // global index of the wave's first root
     uint32_t n_roots;
     unsigned long long *counters;   // [0] closest rays, [1] shadow rays
@@ -194,8 +303,8 @@ struct WaveState {
 // depth limit, an emitter), 1 diffuse only (light samples and the hemisphere ray), 2 a specular
 // or transmitting material (mirror / refraction rays, Whitted.cpp:85-104, PathTracer.cpp:136-157)
 constexpr int kShadeClasses = 3;
-__device__ __forceinline__ uint32_t shade_class(const DevScene &s, const RenderParams &p, const RayRec &rr, uint32_t hit_id) {
-    if (hit_id == MRT_HIT_NONE || rr.depth > p.depth_max) return 0u;
+__device__ __forceinline__ uint32_t shade_class(const DevScene &s, const RenderParams &p, int32_t depth, uint32_t hit_id) {
+    if (hit_id == MRT_HIT_NONE || depth > p.depth_max) return 0u;
     const uint32_t type = MRT_HIT_TYPE(hit_id), i = MRT_HIT_INDEX(hit_id);
     int32_t m = -1;
     if (type == MRT_PRIM_TRIANGLE) m = s.tri_mat[i];
@@ -245,8 +354,8 @@ __device__ __forceinline__ Ray ray_of(const RayRec &r) {
 
 __device__ __forceinline__ Level clamp_level(const WaveState &w, Level L) {
     // a level never reaches past the ray pool (overflowing children were dropped with MRT_ERR_LIMIT)
-    L.start = min(L.start, w.ray_cap);
-    L.count = min(L.count, w.ray_cap - L.start);
+    L.start = min(L.start, w.rec.ray_cap);
+    L.count = min(L.count, w.rec.ray_cap - L.start);
     return L;
 }
 
@@ -293,7 +402,7 @@ __device__ __forceinline__ void shade_ray(const DevScene &s, const RenderParams 
     V3 kd, ks{0, 0, 0}, kt{0, 0, 0};
     float ior = 1.0f;
     if (material_of(s, isect, m)) {
-        if (any_pos(m.le)) { nd.flags = kEmit; nd.point = m.le; return; }
+        if (any_pos(m.le)) { nd.flags = kEmit; nd.kd = m.le; return; }
         kd = m.kd; ks = m.ks; kt = m.kt; ior = m.ior;
     } else {
         kd = isect.color;
@@ -331,21 +440,50 @@ __device__ __forceinline__ void shade_ray(const DevScene &s, const RenderParams 
     o.ior = ior;
 }
 
-// the node record as the resolve pass reads it: a miss or a cut node only its flags, an emitter
-// its radiance, a shaded node its terms with the occlusion and child-flag bits cleared (the
-// children's values arrive from their own resolve)
-__device__ __forceinline__ void store_node(NodeRec &dst, const NodeRec &nd) {
-    dst.flags = nd.flags;
-    const uint32_t kind = nd.flags & 3u;
-    if (kind == kEmit) dst.point = nd.point;
-    if (kind != kShaded) return;
-    dst.occluded = 0;
-    dst.child_flag = 0;
-    dst.kd = nd.kd;
-    dst.ks = nd.ks;
-    dst.kt = nd.kt;
-    dst.point = nd.point;
-    dst.normal = nd.normal;
+// the node record as the resolve pass reads it (the children's values arrive from their own resolve)
+__device__ __forceinline__ void store_node(const WaveRecords &w, uint32_t i, const NodeRec &nd) {
+    uint4 *p = w.nodes + 8 * (size_t)i;
+    store_32b(p, make_uint4(nd.flags, 0u, fbits(nd.kd.x), fbits(nd.kd.y)),
+              make_uint4(fbits(nd.kd.z), fbits(nd.kt.y), fbits(nd.kt.z), 0u));
+    if ((nd.flags & 3u) != kShaded) return;
+    store_32b(p + 2, make_uint4(fbits(nd.point.x), fbits(nd.point.y), fbits(nd.point.z), fbits(nd.normal.x)),
+              make_uint4(fbits(nd.normal.y), fbits(nd.normal.z), fbits(nd.ks.x), fbits(nd.ks.y)));
+    if (nd.flags & (kKsPos | kKtPos)) p[4] = make_uint4(fbits(nd.ks.z), fbits(nd.kt.x), 0u, 0u);
+}
+
+// what resolve_node reads of a node, its children's values included
+__device__ __forceinline__ void load_node(const WaveRecords &w, uint32_t i, NodeRec &nd) {
+    const uint4 *p = w.nodes + 8 * (size_t)i;
+    uint4 a, b;
+    load_32b(p, a, b);
+    nd.flags = a.x;
+    nd.occluded = a.y;
+    nd.kd = V3{bitsf(a.z), bitsf(a.w), bitsf(b.x)};
+    nd.child_flag = 0;
+    if ((nd.flags & 3u) != kShaded) return;
+    const float kty = bitsf(b.y), ktz = bitsf(b.z);
+    load_32b(p + 2, a, b);
+    nd.point = V3{bitsf(a.x), bitsf(a.y), bitsf(a.z)};
+    nd.normal = V3{bitsf(a.w), bitsf(b.x), bitsf(b.y)};
+    const float ksx = bitsf(b.z), ksy = bitsf(b.w);
+    if (nd.flags & kHasIndirect) {
+        const uint4 c = p[6];
+        nd.child[0] = V3{bitsf(c.x), bitsf(c.y), bitsf(c.z)};
+        nd.child_flag = c.w;
+    }
+    if (nd.flags & (kKsPos | kKtPos)) {
+        const uint4 k = p[4], c1 = p[7], c2 = p[5];
+        nd.ks = V3{ksx, ksy, bitsf(k.x)};
+        nd.kt = V3{bitsf(k.y), kty, ktz};
+        nd.child[1] = V3{bitsf(c1.x), bitsf(c1.y), bitsf(c1.z)};
+        nd.child[2] = V3{bitsf(c2.x), bitsf(c2.y), bitsf(c2.z)};
+    }
+}
+
+// a child's value and light flag into its parent's record (the flag is asked for of child 0 only)
+__device__ __forceinline__ void store_child(const WaveRecords &w, uint32_t parent, uint32_t slot, V3 rgb, bool flag) {
+    w.nodes[8 * (size_t)parent + (slot == 2u ? 5u : 6u + slot)] =
+        make_uint4(fbits(rgb.x), fbits(rgb.y), fbits(rgb.z), flag ? 1u : 0u);
 }
 
 // the direction of the continuation ray of `slot` from a shaded node (the hemisphere sample of the
@@ -359,12 +497,12 @@ __device__ __forceinline__ V3 child_dir(const ShadeLane &o, const V3 &d, const S
 
 // the continuation rays in slot order, from the hit point
 __device__ __forceinline__ void emit_children(const DevScene &s, const ShadeLane &o, const RayRec &rr, const Stream &st,
-                                              uint32_t idx, uint32_t pos0, RayRec *rays, uint32_t cap) {
+                                              uint32_t idx, uint32_t pos0, const WaveRecords &w) {
     const V3 d{rr.dx, rr.dy, rr.dz};
     uint32_t pos = pos0;
     for (uint32_t m = o.child_mask; m; m &= m - 1u) {
         const uint32_t slot = (uint32_t)(__ffs(m) - 1);
-        if (pos >= cap) { raise_error(s, MRT_ERR_LIMIT); break; }
+        if (pos >= w.ray_cap) { raise_error(s, MRT_ERR_LIMIT); break; }
         const V3 cd = child_dir(o, d, st, rr.code, slot);
         RayRec q;
         q.ox = o.nd.point.x; q.oy = o.nd.point.y; q.oz = o.nd.point.z;
@@ -375,14 +513,13 @@ __device__ __forceinline__ void emit_children(const DevScene &s, const ShadeLane
         q.parent = idx;
         q.slot = slot;
         q.code = rr.code * 4u + slot + 1u;
-        rays[pos++] = q;
+        store_ray(w, pos++, q);
     }
 }
 
 // the shadow rays of light samples with cos > 0, in light-sample order (Whitted.cpp:33-66)
 __device__ __forceinline__ void emit_shadows(const DevScene &s, const RenderParams &p, const Stream &st, const ShadeLane &o,
-                                             const RayRec &rr, uint32_t idx, uint32_t pos0, ShadowRec *shadows,
-                                             uint32_t cap) {
+                                             const RayRec &rr, uint32_t idx, uint32_t pos0, const WaveRecords &w) {
     if (!o.shaded || o.n_shadow == 0) return;
     uint32_t q = 0;
     for (uint32_t j = 0; j < p.spl; ++j) {
@@ -393,7 +530,7 @@ __device__ __forceinline__ void emit_shadows(const DevScene &s, const RenderPara
         vtl = normalize(vtl);
         if (!(dot(o.nd.normal, vtl) > 0.0f)) continue;
         const uint32_t pos = pos0 + q++;
-        if (pos >= cap) { raise_error(s, MRT_ERR_LIMIT); break; }
+        if (pos >= w.shadow_cap) { raise_error(s, MRT_ERR_LIMIT); break; }
         ShadowRec sr;
         sr.ox = o.nd.point.x; sr.oy = o.nd.point.y; sr.oz = o.nd.point.z;
         sr.dx = vtl.x; sr.dy = vtl.y; sr.dz = vtl.z;
@@ -401,7 +538,7 @@ __device__ __forceinline__ void emit_shadows(const DevScene &s, const RenderPara
         sr.node = idx;
         sr.j = j;
         sr.exclude = o.prim;
-        shadows[pos] = sr;
+        store_shadow(w, pos, sr);
     }
 }
 
@@ -412,7 +549,7 @@ __device__ __forceinline__ void resolve_node(const DevScene &s, const RenderPara
     flag = false;
     const uint32_t kind = nd.flags & 3u;
     if (kind == kEmit) {
-        rgb = nd.point;
+        rgb = nd.kd;
         flag = true;
         return;
     }
