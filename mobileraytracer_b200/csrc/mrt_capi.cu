@@ -318,7 +318,7 @@ static void scene_free(MrtScene *s) {
     DevBuf *bufs[] = {&s->tri_a, &s->tri_ab, &s->tri_ac, &s->tri_n, &s->tri_c, &s->tri_mat, &s->sph, &s->sph_mat,
                       &s->pln_n, &s->pln_p, &s->pln_mat, &s->lights, &s->mats, &s->fnodes, &s->ftris};
     for (DevBuf *b : bufs) dev_free(*b);
-    for (int k = 0; k < 3; ++k) { dev_free(s->rnodes[k]); dev_free(s->grid_start[k]); dev_free(s->grid_refs[k]); }
+    for (int k = 0; k < 3; ++k) { dev_free(s->rnodes[k]); dev_free(s->grid_cells[k]); dev_free(s->grid_refs[k]); }
     dev_free(s->grid_trec);
     for (auto &b : s->work) dev_free(b);
 }
@@ -493,7 +493,7 @@ int mrt_scene_build(MrtScene *s, const MrtAccelOpts *o) {
     s->opts = *o;
     dev_free(s->fnodes);
     dev_free(s->ftris);
-    for (int k = 0; k < 3; ++k) { dev_free(s->rnodes[k]); dev_free(s->grid_start[k]); dev_free(s->grid_refs[k]); }
+    for (int k = 0; k < 3; ++k) { dev_free(s->rnodes[k]); dev_free(s->grid_cells[k]); dev_free(s->grid_refs[k]); }
     dev_free(s->grid_trec);
     s->dev.grid[kTriangle].trec = nullptr;
     s->dev.accel = o->accelerator;
@@ -518,7 +518,7 @@ uint64_t mrt_scene_device_bytes(const MrtScene *s) {
     const DevBuf *bufs[] = {&s->tri_a, &s->tri_ab, &s->tri_ac, &s->tri_n, &s->tri_c, &s->tri_mat, &s->sph, &s->sph_mat,
                             &s->pln_n, &s->pln_p, &s->pln_mat, &s->lights, &s->mats, &s->fnodes, &s->ftris};
     for (const DevBuf *b : bufs) t += b->bytes;
-    for (int k = 0; k < 3; ++k) t += s->rnodes[k].bytes + s->grid_start[k].bytes + s->grid_refs[k].bytes;
+    for (int k = 0; k < 3; ++k) t += s->rnodes[k].bytes + s->grid_cells[k].bytes + s->grid_refs[k].bytes;
     t += s->grid_trec.bytes;
     return t;
 }

@@ -114,6 +114,16 @@ struct RefNode {
     uint32_t count;
 };
 
+// Records of the grid walks, one per cell with a border of one cell around the grid: (first reference, last
+// + 1); (kEmptyCell, d) for an empty cell, d >= 1: every cell at most d - 1 away along each axis is empty
+// and inside the grid; (kEmptyCell, 0) for the border, where a walk ends.
+constexpr uint32_t kEmptyCell = 0xFFFFFFFFu;
+constexpr uint32_t kEmptyReach = 8;           // largest d
+// Skip bits of the triangle grid's references (grids of at most 2^kSkipShift triangles): bit
+// kSkipShift + 2 a + (step < 0) is set when the cell that a walk stepping along axis a comes from lists
+// the triangle too.
+constexpr int kSkipShift = 26;
+
 struct DevGrid {
     int32_t G;
     uint32_t shift;
@@ -121,8 +131,9 @@ struct DevGrid {
     int32_t has;
     V3 mn, mx;          // m_Extends
     V3 sr, cw;          // m_SR, m_CW
-    const uint32_t *start;  // G^3 + 1
-    const uint32_t *refs;
+    const uint2 *cells;     // (G + 2)^3 records, cell (X, Y, Z) at (X + 1) + (Y + 1) (G + 2) + (Z + 1) (G + 2)^2
+    const uint32_t *refs;   // primitive index | skip bits (id_mask takes the index)
+    uint32_t id_mask;
     const float *trec;      // triangle grid: 16 floats per triangle in input order (A, AB, AC, 7 unused),
                             // 64-byte aligned records the walk reads with one 256-bit and one 32-bit load
 };

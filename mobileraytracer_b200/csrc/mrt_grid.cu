@@ -180,12 +180,95 @@ __global__ void k_block_sums(const uint32_t *in, uint64_t n, uint32_t *sums, uin
         sums[blockIdx.x] = t;
     }
 }
-__global__ void k_block_scan_write(const uint32_t *in, uint64_t n, const uint32_t *offsets, uint32_t per, uint32_t *out) {
-    if (threadIdx.x != 0) return;
+// (256 threads a block, 256 counts at a time: one thread per block of 8,192 took 139 us for G = 128)
+__global__ void __launch_bounds__(256) k_block_scan_write(const uint32_t *in, uint64_t n, const uint32_t *offsets, uint32_t per,
+                                                          uint32_t *out) {
+    __shared__ uint32_t wsum[8];
     const uint64_t b = (uint64_t)blockIdx.x * per;
-    uint32_t acc = offsets[blockIdx.x];
-    for (uint64_t i = b; i < b + per && i < n; ++i) { out[i] = acc; acc += in[i]; }
-    if (b + per >= n && b < n) out[n] = acc;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t carry = offsets[blockIdx.x];
+    for (uint64_t i0 = b; i0 < b + per && i0 < n; i0 += 256) {
+        const uint64_t i = i0 + threadIdx.x;
+        const uint32_t v = i < n ? in[i] : 0u;
+        uint32_t incl = v;
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t w = __shfl_up_sync(0xFFFFFFFFu, incl, o);
+            if (lane >= o) incl += w;
+        }
+        if (lane == 31) wsum[warp] = incl;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+        for (int w = 0; w < 8; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (i < n) out[i] = carry + before + incl - v;
+        carry += all;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0 && b + per >= n && b < n) out[n] = carry;
+}
+
+// --- what the walks read (mrt_gridwalk.cuh) -----------------------------------------------------------
+// A walk's cell (X, Y, Z) reads the list at X + Y sy + Z sz (RegularGrid.hpp:237-241; sy and sz by the
+// addressing mode).
+struct WalkCells {
+    uint32_t G;
+    uint64_t sy, sz;
+    const uint32_t *start;
+    // padded record i: false for the border, else the list's ends
+    __device__ bool list(uint64_t i, uint32_t &b, uint32_t &e) const {
+        const uint32_t p = G + 2u, x = (uint32_t)(i % p), y = (uint32_t)(i / p % p), z = (uint32_t)(i / ((uint64_t)p * p));
+        if (x == 0 || y == 0 || z == 0 || x > G || y > G || z > G) return false;
+        const uint64_t c = (x - 1u) + (y - 1u) * sy + (z - 1u) * sz;
+        b = start[c];
+        e = start[c + 1];
+        return true;
+    }
+};
+// reach: 0 for the border and for a cell that lists something, d for one whose surroundings are empty up to
+// d - 1 cells away
+__global__ void k_reach_init(uint64_t n, WalkCells w, uint8_t *reach) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    uint32_t b, e;
+    if (i < n) reach[i] = w.list(i, b, e) && b == e ? 1 : 0;
+}
+// d - 1 -> d where the cell and its 26 neighbours are at d - 1 (or at d already), in place
+__global__ void k_reach_grow(uint64_t n, int64_t p, uint32_t d, uint8_t *reach) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || reach[i] != d - 1) return;   // (the border stays 0: the cells left have all 26)
+    for (int64_t z = -1; z <= 1; ++z)
+        for (int64_t y = -1; y <= 1; ++y)
+            for (int64_t x = -1; x <= 1; ++x)
+                if (reach[(int64_t)i + x + (y + z * p) * p] < d - 1) return;
+    reach[i] = (uint8_t)d;
+}
+__global__ void k_write_cells(uint64_t n, WalkCells w, const uint8_t *__restrict__ reach, uint2 *cells) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t b = 0, e = 0;
+    const bool inside = w.list(i, b, e);
+    cells[i] = inside && b < e ? make_uint2(b, e) : make_uint2(kEmptyCell, reach[i]);
+}
+// skip bits: each list against the lists of the six cells a walk can come from (both in ascending order)
+__global__ void k_skip_bits(int64_t ncell, int64_t sy, int64_t sz, const uint32_t *__restrict__ start, uint32_t *refs) {
+    const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (c >= ncell) return;
+    const uint32_t b = start[c], e = start[c + 1], mask = (1u << kSkipShift) - 1u;
+    if (b == e) return;
+    const int64_t stride[3] = {1, sy, sz};
+    for (int k = 0; k < 6; ++k) {
+        const int64_t from = (k & 1) ? c + stride[k >> 1] : c - stride[k >> 1];
+        if (from < 0 || from >= ncell) continue;
+        uint32_t i = b, j = start[from];
+        const uint32_t je = start[from + 1];
+        while (i < e && j < je) {
+            const uint32_t u = refs[i] & mask, v = refs[j] & mask;
+            if (u == v) refs[i] |= 1u << (kSkipShift + k);   // only this thread writes its cell's references
+            if (u <= v) ++i;
+            if (v <= u) ++j;
+        }
+    }
 }
 
 uint32_t bit_counter(uint32_t n) { uint32_t c = 0; while (n > 0) { ++c; n >>= 1; } return c; }   // Utils.cpp:26-33
@@ -297,8 +380,8 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
         p.rx = p.dx > 0 ? 1.0f / p.dx : 1.0f;
         p.ry = p.dy > 0 ? 1.0f / p.dy : 1.0f;
         p.rz = p.dz > 0 ? 1.0f / p.dz : 1.0f;
-        int st = dev_alloc(ctx, s->grid_start[type], 4ull * (ncell + 1));
-        DevBuf count, fill, sums, offs;
+        DevBuf start_buf, count, fill, sums, offs, reach;
+        int st = dev_alloc(ctx, start_buf, 4ull * (ncell + 1));
         const uint32_t per = 8192;
         const uint64_t nblk = (ncell + per - 1) / per;
         if (st == MRT_OK) st = dev_alloc(ctx, count, 4ull * ncell);
@@ -320,12 +403,12 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
             if (st == MRT_OK && total > 0xFFFFFFF0ull) { set_error(ctx, "grid: more than 2^32 references"); st = MRT_ERR_LIMIT; }
             if (st == MRT_OK) st = cuda_status(ctx, cudaMemcpyAsync(offs.ptr, ho.data(), 4ull * nblk, cudaMemcpyHostToDevice, q), "grid offs");
             if (st == MRT_OK) {
-                k_block_scan_write<<<(uint32_t)nblk, 32, 0, q>>>((const uint32_t *)count.ptr, ncell, (const uint32_t *)offs.ptr,
-                                                                per, (uint32_t *)s->grid_start[type].ptr);
+                k_block_scan_write<<<(uint32_t)nblk, 256, 0, q>>>((const uint32_t *)count.ptr, ncell, (const uint32_t *)offs.ptr,
+                                                                per, (uint32_t *)start_buf.ptr);
                 st = dev_alloc(ctx, s->grid_refs[type], 4ull * (total ? total : 1));
             }
             if (st == MRT_OK) {
-                const uint32_t *start = (const uint32_t *)s->grid_start[type].ptr;
+                const uint32_t *start = (const uint32_t *)start_buf.ptr;
                 uint32_t *refs = (uint32_t *)s->grid_refs[type].ptr;
                 if (type == kTriangle) launch_fill<kTriangle>(s, p, n, nullptr, start, (uint32_t *)fill.ptr, refs, 1);
                 else if (type == kSphere) launch_fill<kSphere>(s, p, n, nullptr, start, (uint32_t *)fill.ptr, refs, 1);
@@ -337,8 +420,30 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
             }
         }
         dev_free(count); dev_free(fill); dev_free(sums); dev_free(offs);
+        // the cell records and the skip bits, along the strides the walks read with
+        g.id_mask = 0xFFFFFFFFu;
+        const uint64_t padded = (uint64_t)(G + 2) * (uint64_t)(G + 2) * (uint64_t)(G + 2);
+        if (st == MRT_OK) st = dev_alloc(ctx, s->grid_cells[type], sizeof(uint2) * padded);
+        if (st == MRT_OK) st = dev_alloc(ctx, reach, padded);
+        if (st == MRT_OK) {
+            const uint32_t *start = (const uint32_t *)start_buf.ptr;
+            const bool linear = grid_index == MRT_GRID_INDEX_LINEAR;
+            const int64_t sy = linear ? (int64_t)G : (int64_t)1 << g.shift, sz = linear ? (int64_t)G * G : (int64_t)1 << (2 * g.shift);
+            const WalkCells wc{(uint32_t)G, (uint64_t)sy, (uint64_t)sz, start};
+            const uint32_t blocks = (uint32_t)((ncell + 255) / 256), pblocks = (uint32_t)((padded + 255) / 256);
+            k_reach_init<<<pblocks, 256, 0, q>>>(padded, wc, (uint8_t *)reach.ptr);
+            for (uint32_t d = 2; d <= kEmptyReach; ++d) k_reach_grow<<<pblocks, 256, 0, q>>>(padded, (int64_t)G + 2, d, (uint8_t *)reach.ptr);
+            k_write_cells<<<pblocks, 256, 0, q>>>(padded, wc, (const uint8_t *)reach.ptr, (uint2 *)s->grid_cells[type].ptr);
+            if (type == kTriangle && n <= 1u << kSkipShift) {
+                k_skip_bits<<<blocks, 256, 0, q>>>((int64_t)ncell, sy, sz, start, (uint32_t *)s->grid_refs[type].ptr);
+                g.id_mask = (1u << kSkipShift) - 1u;
+            }
+            st = cuda_status(ctx, cudaGetLastError(), "grid cells");
+            if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "grid cells");
+        }
+        dev_free(start_buf); dev_free(reach);
         if (st != MRT_OK) return st;
-        g.start = (const uint32_t *)s->grid_start[type].ptr;
+        g.cells = (const uint2 *)s->grid_cells[type].ptr;
         g.refs = (const uint32_t *)s->grid_refs[type].ptr;
         g.trec = nullptr;
         if (type == kTriangle && n > 0 && kGridTriRecords) {

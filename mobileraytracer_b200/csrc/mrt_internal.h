@@ -77,7 +77,7 @@ struct MrtScene {
     uint64_t fnode_count = 0;
     DevBuf rnodes[3];
     uint64_t rnode_count[3] = {0, 0, 0};
-    DevBuf grid_start[3], grid_refs[3], grid_trec;
+    DevBuf grid_cells[3], grid_refs[3], grid_trec;
     uint64_t grid_refs_count[3] = {0, 0, 0};
     // host copies needed by the reference-tree build and the grid bounds
     std::vector<float> h_abc;           // 9 floats per triangle

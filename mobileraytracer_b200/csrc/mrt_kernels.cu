@@ -114,6 +114,11 @@ __global__ void __launch_bounds__(128, kGridBlocksPerSm) k_trace_grid_persistent
     persistent_grid_closest(s, work, lane);
 }
 
+__global__ void __launch_bounds__(128, kGridBlocksPerSm) k_trace_any_grid(DevScene s, AnyWork work) {
+    TraceLane lane;
+    persistent_grid_any(s, work, lane);
+}
+
 // counting replay of the grid closest hit: planes and spheres in order, then the triangle grid
 // (counted: cells visited and triangle references tested), as k_trace_closest
 __global__ void __launch_bounds__(128) k_trace_counts_grid(DevScene s, const MrtRay *rays, uint32_t n, uint32_t *cells,
@@ -189,6 +194,12 @@ int launch_trace_any(MrtScene *s, const MrtRay *d_rays, const float *d_dist, uin
         AnyWork w{d_rays, d_dist, d_occ, n, ctx->d_counters};
         k_trace_any_persistent<<<persistent_grid(ctx, n), 128, 0, ctx->stream>>>(s->dev, w);
         return cuda_status(ctx, cudaGetLastError(), "k_trace_any_persistent");
+    }
+    if (s->opts.accelerator == MRT_ACCEL_REGULAR_GRID) {
+        cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), ctx->stream);
+        AnyWork w{d_rays, d_dist, d_occ, n, ctx->d_counters};
+        k_trace_any_grid<<<persistent_grid(ctx, n), 128, 0, ctx->stream>>>(s->dev, w);
+        return cuda_status(ctx, cudaGetLastError(), "k_trace_any_grid");
     }
     MRT_DISPATCH(launch_any, s->opts.accelerator, s->opts.bvh_mode, s->dev, d_rays, d_dist, n, d_occ, grid_for(ctx, n), ctx->stream);
     return cuda_status(ctx, cudaGetLastError(), "k_trace_any");

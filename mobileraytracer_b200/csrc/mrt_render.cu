@@ -489,6 +489,14 @@ __global__ void __launch_bounds__(128, kWaveBlocksPerSm) k_wave_shadow_fast(DevS
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[1], (unsigned long long)n);
 }
 
+__global__ void __launch_bounds__(128, kGridBlocksPerSm) k_wave_shadow_grid(DevScene s, WaveState w, int level, uint32_t *ctr) {
+    const uint32_t n = min(w.levels[level].shadow_count, w.rec.shadow_cap);
+    ShadowWork work{w, n, ctr};
+    WaveLane lane;
+    persistent_grid_any(s, work, lane);
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[1], (unsigned long long)n);
+}
+
 // whole camera paths in one persistent launch (mrt_paths.cuh): work item = the wave's path i
 struct WavePathWork {
     const DevScene *s;
@@ -687,7 +695,8 @@ void launch_wave_level(const DevScene &s, const RenderParams &p, const WaveState
     else k_wave_extend<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
     if (w.sort_shading) k_wave_shade_sorted<<<grid, 128, 0, q>>>(s, p, w, level);
     else k_wave_shade<<<grid, 128, 0, q>>>(s, p, w, level);
-    k_wave_shadow<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
+    if (ACCEL == MRT_ACCEL_REGULAR_GRID) k_wave_shadow_grid<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level + 1);
+    else k_wave_shadow<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
 }
 
 #define MRT_DISPATCH(fn, accel, mode, ...)                                                                 \

@@ -225,10 +225,16 @@ struct Dda {
     float tx, ty, tz, dx, dy, dz;
 };
 
+// the record of a cell (the addressing modes differ in the list that the build put there)
 __device__ __forceinline__ uint32_t grid_cell(const DevGrid &g, int32_t X, int32_t Y, int32_t Z) {
-    if (g.index_mode == MRT_GRID_INDEX_LINEAR)
-        return (uint32_t)X + (uint32_t)Y * (uint32_t)g.G + (uint32_t)Z * (uint32_t)g.G * (uint32_t)g.G;
-    return (uint32_t)X + ((uint32_t)Y << g.shift) + ((uint32_t)Z << (g.shift * 2u));
+    const uint32_t p = (uint32_t)g.G + 2u;
+    return (uint32_t)(X + 1) + ((uint32_t)(Y + 1) + (uint32_t)(Z + 1) * p) * p;
+}
+// its references: refs[b .. e)
+__device__ __forceinline__ void grid_list(const DevGrid &g, uint32_t c, uint32_t &b, uint32_t &e) {
+    const uint2 r = __ldg(&g.cells[c]);
+    b = r.x == kEmptyCell ? 0u : r.x;
+    e = r.x == kEmptyCell ? 0u : r.y;
 }
 
 // DDA setup, RegularGrid.hpp:161-231
@@ -266,7 +272,7 @@ __device__ __forceinline__ bool dda_step(Dda &s) {
     return true;
 }
 
-// cells visited (start[c], start[c + 1] read) and references tested (refs[k] and the primitive read)
+// cells visited (cell record read) and references tested (refs[k] and the primitive read)
 struct GridCounts {
     uint32_t cells;
     uint32_t refs;
@@ -282,12 +288,13 @@ __device__ bool grid_trace(const DevScene &s, const Ray &r, float &len, uint32_t
     uint32_t steps = 0;
     for (;;) {
         const uint32_t c = grid_cell(g, st.X, st.Y, st.Z);
-        const uint32_t b = g.start[c], e = g.start[c + 1];
+        uint32_t b, e;
+        grid_list(g, c, b, e);
         if (kCount) cnt->cells++;
         bool found = false;
         for (uint32_t k = b; k < e; ++k) {
             if (kCount) cnt->refs++;
-            hit |= prim_hit<T>(s, g.refs[k], r, len, id);
+            hit |= prim_hit<T>(s, g.refs[k] & g.id_mask, r, len, id);
             if (hit) { found = true; break; }
         }
         if (found) break;
@@ -296,9 +303,10 @@ __device__ bool grid_trace(const DevScene &s, const Ray &r, float &len, uint32_t
     }
     for (;;) {   // testloop, RegularGrid.hpp:282-335
         const uint32_t c = grid_cell(g, st.X, st.Y, st.Z);
-        const uint32_t b = g.start[c], e = g.start[c + 1];
+        uint32_t b, e;
+        grid_list(g, c, b, e);
         if (kCount) { cnt->cells++; cnt->refs += e - b; }
-        for (uint32_t k = b; k < e; ++k) hit |= prim_hit<T>(s, g.refs[k], r, len, id);
+        for (uint32_t k = b; k < e; ++k) hit |= prim_hit<T>(s, g.refs[k] & g.id_mask, r, len, id);
         if (st.tx < st.ty) {
             if (st.tx < st.tz) {
                 if (len < st.tx) break;
@@ -330,9 +338,10 @@ __device__ bool grid_occ(const DevScene &s, const Ray &r, float dist) {
     uint32_t steps = 0;
     for (;;) {
         const uint32_t c = grid_cell(g, st.X, st.Y, st.Z);
-        const uint32_t b = g.start[c], e = g.start[c + 1];
+        uint32_t b, e;
+        grid_list(g, c, b, e);
         for (uint32_t k = b; k < e; ++k)
-            if (prim_occ<T>(s, g.refs[k], r, dist)) return true;
+            if (prim_occ<T>(s, g.refs[k] & g.id_mask, r, dist)) return true;
         if (!dda_step(st)) return false;
         if (++steps > kMaxGridSteps) { raise_error(s, MRT_ERR_LIMIT); return false; }
     }
