@@ -41,7 +41,11 @@ def _after_torch(ctx, *tensors):
     queued on its current stream (e.g. the zeroing or upload of a device buffer passed in)."""
     if any(_is_torch_cuda(t) for t in tensors if t is not None):
         import torch
-        torch.cuda.ExternalStream(ctx.stream).wait_stream(torch.cuda.current_stream())
+        current = torch.cuda.current_stream()
+        if not current.query():   # nothing queued: nothing to wait for
+            if ctx._torch_stream is None:
+                ctx._torch_stream = torch.cuda.ExternalStream(ctx.stream)
+            ctx._torch_stream.wait_stream(current)
 
 
 def _ptr(x):
@@ -63,6 +67,7 @@ class Context:
             raise MrtError(st, f"mrt_context_create(device={device}) failed")
         self.h = h
         self.device = device
+        self._torch_stream = None   # the context's stream as torch sees it
         self._scenes = weakref.WeakSet()
         self._batches = weakref.WeakSet()
 

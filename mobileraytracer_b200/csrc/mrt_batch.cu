@@ -862,6 +862,8 @@ int mrt_batch_create(MrtContext *ctx, const MrtBatchOpts *opts, MrtBatch **out) 
     if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreateWithFlags(&b->ev_jobs, cudaEventDisableTiming), "cudaEventCreate");
     if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreate(&b->ev_first), "cudaEventCreate");
     if (st == MRT_OK) st = cuda_status(ctx, cudaMemsetAsync(b->d_counters.ptr, 0, 4 * sizeof(unsigned long long), ctx->stream), "memset");
+    // the pipelines' streams use the buffers: wait for their allocation on the context's stream
+    if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_batch_create");
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_batch_create");
     if (st != MRT_OK) { free_batch(b); return st; }
     *out = b;

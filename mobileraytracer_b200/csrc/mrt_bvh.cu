@@ -758,14 +758,15 @@ int build_fast_bvh(MrtScene *s) {
 
 int build_reference_bvh(MrtScene *s) {
     MrtContext *ctx = s->ctx;
+    const int got = host_triangles(s);
+    if (got != MRT_OK) return got;
     for (int k = 0; k < 3; ++k) {
         std::vector<HBox> boxes;
         if (k == kTriangle) {
             boxes.resize(s->n_tri);
             for (uint32_t i = 0; i < s->n_tri; ++i) {   // Triangle::getAABB, Triangle.cpp:145-152
-                const float *p = &s->h_abc[9ull * i];
-                const V3 A{p[0], p[1], p[2]};
-                const V3 ab = V3{p[3], p[4], p[5]} - A, ac = V3{p[6], p[7], p[8]} - A;
+                const float *p = &s->h_tri[9ull * i];
+                const V3 A{p[0], p[1], p[2]}, ab{p[3], p[4], p[5]}, ac{p[6], p[7], p[8]};
                 const V3 B = A + ab, C = A + ac;
                 boxes[i] = HBox{vmin(A, vmin(B, C)), vmax(A, vmax(B, C))};
             }

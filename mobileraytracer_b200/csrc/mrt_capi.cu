@@ -77,6 +77,55 @@ static void arena_free(MrtArena *a, void *p, size_t bytes) {
     --a->live;
 }
 
+// Buffers below kPoolMost come from one memory pool per device, shared by its contexts (thread-safe) and
+// made with the first of them.  Opening a scene allocates and frees some 45 buffers; with cudaMalloc and
+// cudaFree, each of which maps memory and waits for the device, a 200,003-triangle scene took 16 to 57 ms
+// to upload, build and render once, of which the kernels are 0.9 ms.  The pool keeps at most kPoolKeep
+// unused bytes (trim_pool, after builds and when scenes go) and none once the device's last context is
+// gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight (for a pooled
+// buffer cudaFree does not wait).  Larger buffers are few and long-lived (ray pools) and would only make the
+// pool's bound meaningless.
+constexpr size_t kPoolMost = 256u << 20, kPoolKeep = 1u << 30;
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+};
+std::mutex g_pool_mu;
+std::map<int, DevicePool> g_pools;
+
+int pool_join(MrtContext *ctx) {
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool &d = g_pools[ctx->device];
+    if (!d.pool) {
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.handleTypes = cudaMemHandleTypeNone;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        const int st = cuda_status(ctx, cudaMemPoolCreate(&d.pool, &props), "cudaMemPoolCreate");
+        if (st != MRT_OK) { d.pool = nullptr; return st; }
+        uint64_t keep = ~0ull;   // nothing is given back by itself: trim_pool bounds what is unused
+        cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    }
+    ctx->pool = d.pool;
+    ++d.contexts;
+    return MRT_OK;
+}
+void pool_leave(MrtContext *ctx) {
+    if (!ctx->pool) return;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    DevicePool &d = g_pools[ctx->device];
+    if (--d.contexts == 0) cudaMemPoolTrimTo(d.pool, 0);
+    ctx->pool = nullptr;
+}
+void trim_pool(MrtContext *ctx) {
+    uint64_t reserved = 0, used = 0;
+    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
+        return;
+    if (reserved - used > kPoolKeep) cudaMemPoolTrimTo(ctx->pool, (size_t)used + kPoolKeep);
+}
+
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
     dev_free(b);
     if (bytes == 0) bytes = 16;
@@ -96,7 +145,20 @@ int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
         b.arena = ctx->arena;
         return MRT_OK;
     }
-    const cudaError_t e = cudaMalloc(&b.ptr, bytes);
+    cudaError_t e = cudaErrorMemoryAllocation;
+    if (ctx->pool && bytes < kPoolMost) {
+        e = cudaMallocFromPoolAsync(&b.ptr, bytes, ctx->pool, ctx->stream);
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            cudaMemPoolTrimTo(ctx->pool, 0);
+        }
+    }
+    if (e != cudaSuccess) e = cudaMalloc(&b.ptr, bytes);
+    if (e == cudaErrorMemoryAllocation && ctx->pool) {   // what the pool keeps unused may be what is missing
+        cudaGetLastError();
+        cudaMemPoolTrimTo(ctx->pool, 0);
+        e = cudaMalloc(&b.ptr, bytes);
+    }
     if (e != cudaSuccess) {
         b.ptr = nullptr;
         cudaGetLastError();
@@ -123,14 +185,32 @@ int ensure(MrtContext *ctx, DevBuf &b, size_t bytes) {
 }
 
 int check_kernel_error(MrtContext *ctx) {
-    int32_t flag = 0;
-    cudaError_t e = cudaMemcpyAsync(&flag, ctx->d_error, sizeof(flag), cudaMemcpyDeviceToHost, ctx->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e != cudaSuccess) return cuda_status(ctx, e, "kernel");
+    const int st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "kernel");
+    if (st != MRT_OK) return st;
+    const int32_t flag = *const_cast<volatile int32_t *>(&ctx->status->error);
     if (flag != 0) {
-        cudaMemsetAsync(ctx->d_error, 0, sizeof(int32_t), ctx->stream);
+        ctx->status->error = 0;
         set_error(ctx, "a traversal cap was exceeded (stack or step limit)");
         return flag;
+    }
+    return MRT_OK;
+}
+
+int host_triangles(MrtScene *s) {
+    const size_t n = s->n_tri;
+    if (s->h_tri.size() == 9 * n) return MRT_OK;
+    std::vector<float4> part(n);
+    s->h_tri.resize(9 * n);
+    const DevBuf *src[3] = {&s->tri_a, &s->tri_ab, &s->tri_ac};
+    for (int k = 0; k < 3; ++k) {
+        int st = cuda_status(s->ctx, cudaMemcpyAsync(part.data(), src[k]->ptr, 16ull * n, cudaMemcpyDeviceToHost, s->ctx->stream), "triangles");
+        if (st == MRT_OK) st = cuda_status(s->ctx, cudaStreamSynchronize(s->ctx->stream), "triangles");
+        if (st != MRT_OK) { s->h_tri.clear(); return st; }
+        for (size_t i = 0; i < n; ++i) {
+            s->h_tri[9 * i + 3 * k] = part[i].x;
+            s->h_tri[9 * i + 3 * k + 1] = part[i].y;
+            s->h_tri[9 * i + 3 * k + 2] = part[i].z;
+        }
     }
     return MRT_OK;
 }
@@ -212,9 +292,15 @@ int mrt_context_create(int device, MrtContext **out) {
     int st = cuda_status(ctx, cudaSetDevice(device), "cudaSetDevice");
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking), "stream");
     if (st == MRT_OK) st = cuda_status(ctx, cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device), "attr");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaMalloc(&ctx->d_error, sizeof(int32_t)), "cudaMalloc");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaMemset(ctx->d_error, 0, sizeof(int32_t)), "memset");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaMalloc(&ctx->d_counters, 64 * sizeof(uint32_t)), "cudaMalloc");
+    if (st == MRT_OK) st = cuda_status(ctx, cudaHostAlloc(&ctx->status, sizeof(MrtContext::Status), cudaHostAllocMapped), "cudaHostAlloc");
+    if (st == MRT_OK) {
+        *ctx->status = MrtContext::Status{};
+        void *dev = nullptr;
+        st = cuda_status(ctx, cudaHostGetDevicePointer(&dev, &ctx->status->error, 0), "cudaHostGetDevicePointer");
+        ctx->d_error = (int32_t *)dev;
+    }
+    if (st == MRT_OK) st = cuda_status(ctx, cudaMalloc(&ctx->d_counters, MrtContext::kWorkCounters * sizeof(uint32_t) + 2 * sizeof(unsigned long long)), "cudaMalloc");
+    if (st == MRT_OK) st = pool_join(ctx);
     if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreate(&ctx->ev0), "event");
     if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreate(&ctx->ev1), "event");
     for (auto &e : ctx->trace_ev)
@@ -242,8 +328,9 @@ void mrt_context_destroy(MrtContext *ctx) {
     for (auto &b : ctx->scratch) dev_free(b);
     for (auto &b : ctx->wave) dev_free(b);
     for (auto &b : ctx->raster) dev_free(b);
-    if (ctx->d_error) cudaFree(ctx->d_error);
+    if (ctx->status) cudaFreeHost(ctx->status);
     if (ctx->d_counters) cudaFree(ctx->d_counters);
+    pool_leave(ctx);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->ev1) cudaEventDestroy(ctx->ev1);
     for (auto &e : ctx->trace_ev) if (e) cudaEventDestroy(e);
@@ -438,7 +525,6 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
     up(s->lights, hl.data(), sizeof(DevLight) * s->n_light);
     up(s->mats, hm.data(), sizeof(DevMaterial) * s->n_mat);
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "scene upload");
-    s->h_abc.assign(d->tri_abc, d->tri_abc + 9ull * nt);
     dev_free(st_abc); dev_free(st_n); dev_free(st_c); dev_free(st_m);
     if (st != MRT_OK) {
         if (ctx->error.empty()) set_error(ctx, "mrt_scene_create: invalid light kind");
@@ -463,6 +549,7 @@ void mrt_scene_destroy(MrtScene *s) {
     cudaSetDevice(s->ctx->device);
     cudaStreamSynchronize(s->ctx->stream);
     scene_free(s);
+    trim_pool(s->ctx);
     delete s;
 }
 
@@ -508,6 +595,7 @@ int mrt_scene_build(MrtScene *s, const MrtAccelOpts *o) {
     }
     if (st != MRT_OK) return st;
     st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_scene_build");
+    trim_pool(ctx);
     if (st == MRT_OK) s->built = true;
     return st;
 }

@@ -287,9 +287,8 @@ struct HostBox {
 
 HostBox host_prim_box(const MrtScene *s, int type, uint32_t i) {
     if (type == kTriangle) {
-        const float *p = &s->h_abc[9ull * i];
-        const V3 A{p[0], p[1], p[2]};
-        const V3 ab = V3{p[3], p[4], p[5]} - A, ac = V3{p[6], p[7], p[8]} - A;
+        const float *p = &s->h_tri[9ull * i];
+        const V3 A{p[0], p[1], p[2]}, ab{p[3], p[4], p[5]}, ac{p[6], p[7], p[8]};
         const V3 B = A + ab, C = A + ac;
         return HostBox{vmin(A, vmin(B, C)), vmax(A, vmax(B, C))};
     }
@@ -346,6 +345,8 @@ namespace mrt_host {
 int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int grid_size, int grid_index) {
     MrtContext *ctx = s->ctx;
     cudaStream_t q = ctx->stream;
+    const int got = host_triangles(s);
+    if (got != MRT_OK) return got;
     for (int type = 0; type < 3; ++type) {
         const uint32_t n = type == kTriangle ? s->n_tri : (type == kSphere ? s->n_sph : s->n_pln);
         // Scene::getBounds (Scene.cpp:42-45) over the primitives, then the camera (Camera.cpp:39-44)

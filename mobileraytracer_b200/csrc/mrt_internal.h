@@ -40,8 +40,20 @@ struct MrtContext {
     cudaStream_t stream = nullptr;
     std::string error;
     int sm_count = 148;
-    int32_t *d_error = nullptr;         // device error flag (MRT_ERR_LIMIT from kernels)
-    uint32_t *d_counters = nullptr;     // work counters of the persistent kernels (64 slots)
+    // Page-locked host memory that kernels and small copies write and the host reads once the stream is
+    // done, without a copy of its own to wait for.
+    struct Status {
+        int32_t error;                  // MRT_ERR_LIMIT from kernels, the only code they raise
+        int32_t pad;
+        unsigned long long count[4];    // a call's counters
+    };
+    Status *status = nullptr;           // host address
+    int32_t *d_error = nullptr;         // device address of status->error
+    // work counters of the persistent kernels (64 slots), then the two ray counters of a render
+    uint32_t *d_counters = nullptr;
+    static constexpr int kWorkCounters = 64;
+    unsigned long long *ray_counters() const { return reinterpret_cast<unsigned long long *>(d_counters + kWorkCounters); }
+    cudaMemPool_t pool = nullptr;       // the device's pool (mrt_capi.cu)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     static constexpr int kTraceEvents = 16;             // start / end pairs around traversal launches
     cudaEvent_t trace_ev[2 * kTraceEvents] = {};
@@ -80,7 +92,7 @@ struct MrtScene {
     DevBuf grid_cells[3], grid_refs[3], grid_trec;
     uint64_t grid_refs_count[3] = {0, 0, 0};
     // host copies needed by the reference-tree build and the grid bounds
-    std::vector<float> h_abc;           // 9 floats per triangle
+    std::vector<float> h_tri;           // A, AB, AC per triangle (host_triangles; empty until a build asks for it)
     std::vector<float> h_sph;           // 4 per sphere
     std::vector<float> h_pln;           // 6 per plane (point, normalised normal)
     // render state
@@ -101,7 +113,11 @@ int cuda_status(MrtContext *ctx, cudaError_t e, const char *what);
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int ensure(MrtContext *ctx, DevBuf &b, size_t bytes);   // grow-only scratch
-int check_kernel_error(MrtContext *ctx);                // reads and clears the device error flag
+int check_kernel_error(MrtContext *ctx);                // waits for the stream, reads and clears the error flag
+void trim_pool(MrtContext *ctx);                        // gives memory beyond the pool's bound back
+
+// the triangles' A, AB, AC as the device has them in s->h_tri (the reference tree and the grid bounds need them)
+int host_triangles(MrtScene *s);
 
 // builds (mrt_bvh.cu, mrt_grid.cu)
 int build_fast_bvh(MrtScene *s);

@@ -520,9 +520,10 @@ extern "C" int mrt_raster_preview(MrtScene *s, const MrtCamera *cam, uint32_t wi
     k_raster_resolve<<<grid, 256, 0, q>>>(s->dev, p, d_bitmap, stride_bytes / 4u);
     cudaEventRecord(ctx->ev1, q);
     st = cuda_status(ctx, cudaGetLastError(), "raster kernels");
-    unsigned long long counts[4] = {0, 0, 0, 0};
+    unsigned long long *counts = ctx->status->count;   // page-locked: the copy is queued, one wait for all
+    const size_t counts_bytes = 4 * sizeof(unsigned long long);
     if (st == MRT_OK)
-        st = cuda_status(ctx, cudaMemcpyAsync(counts, p.counts, sizeof(counts), cudaMemcpyDeviceToHost, q), "raster counts");
+        st = cuda_status(ctx, cudaMemcpyAsync(counts, p.counts, counts_bytes, cudaMemcpyDeviceToHost, q), "raster counts");
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "raster preview");
     // triangles sent on by a full queue: further passes over the overflow list (only scenes whose
     // large pieces exceed the queue), the image resolved again after each
@@ -538,12 +539,13 @@ extern "C" int mrt_raster_preview(MrtScene *s, const MrtCamera *cam, uint32_t wi
         k_raster_resolve<<<grid, 256, 0, q>>>(s->dev, p, d_bitmap, stride_bytes / 4u);
         st = cuda_status(ctx, cudaGetLastError(), "raster kernels");
         if (st == MRT_OK)
-            st = cuda_status(ctx, cudaMemcpyAsync(counts, p.counts, sizeof(counts), cudaMemcpyDeviceToHost, q), "raster counts");
+            st = cuda_status(ctx, cudaMemcpyAsync(counts, p.counts, counts_bytes, cudaMemcpyDeviceToHost, q), "raster counts");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "raster preview");
     }
-    if (st == MRT_OK && mem == MRT_MEM_HOST)
+    if (st == MRT_OK && mem == MRT_MEM_HOST) {
         st = cuda_status(ctx, cudaMemcpyAsync(bitmap, d_bitmap, bm_bytes, cudaMemcpyDeviceToHost, q), "bitmap out");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "raster preview");
+        if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "raster preview");
+    }
     if (st != MRT_OK) return st;
     if (stats) {
         float ms = 0.0f;

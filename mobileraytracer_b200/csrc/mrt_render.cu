@@ -866,6 +866,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
     }
     const int grid = ctx->sm_count * 16;
     uint64_t rays_closest = 0, rays_shadow = 0;
+    bool counted = false;    // the kernels count the rays
     uint32_t launches = 0;   // kernels launched by this render
     float trace_ms = 0.0f;
     int trace_pairs = 0;   // recorded pairs of ctx->trace_ev not yet added to trace_ms
@@ -1007,16 +1008,16 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         }
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[4], sizeof(Level) * (levels + 2));
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[5], sizeof(float4) * wave);
-        if (st == MRT_OK) st = ensure(ctx, ctx->wave[6], 16);
         if (st != MRT_OK) return st;
         WaveState w{};
         w.rec = wave_records(ctx->wave[1].ptr, ctx->wave[2].ptr, ctx->wave[3].ptr, (uint32_t)ray_cap, (uint32_t)shadow_cap);
         w.levels = (Level *)ctx->wave[4].ptr;
         w.root_rgb = (float4 *)ctx->wave[5].ptr;
-        w.counters = (unsigned long long *)ctx->wave[6].ptr;
+        w.counters = ctx->ray_counters();
         // per-material shade queues where the scene mixes diffuse with mirror / glass materials
         w.sort_shading = (o->flags & MRT_RENDER_SHADE_QUEUES) && s->mixed_materials ? 1u : 0u;
-        cudaMemsetAsync(w.counters, 0, 16, q);
+        // the work counters of the first wave and the ray counters
+        cudaMemsetAsync(ctx->d_counters, 0, MrtContext::kWorkCounters * sizeof(uint32_t) + 16, q);
         // at most one wave queued ahead of the one running: a stop request ends the render within two
         // waves, and progress counts finished waves
         uint64_t waves_issued = 0;
@@ -1035,12 +1036,12 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 w.root_first = (uint32_t)r0;
                 w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
                 if (paths) {
-                    cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
+                    if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
                     k_wave_paths<<<ctx->sm_count * 8, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
                     launches += 2;   // with the fold below
                 } else {
                     cudaMemsetAsync(w.levels, 0, sizeof(Level) * (levels + 2), q);
-                    cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t) * 2 * (levels + 1), q);
+                    if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t) * 2 * (levels + 1), q);
                     k_wave_raygen<<<grid, 128, 0, q>>>(p, w);
                     for (int b = 0; b < levels; ++b)
                         MRT_DISPATCH(launch_wave_level, accel, mode, s->dev, p, w, b, grid, q, ctx->d_counters);
@@ -1055,16 +1056,18 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 ++waves_issued;
             }
         }
-        unsigned long long cnt[2] = {0, 0};
-        st = cuda_status(ctx, cudaMemcpyAsync(cnt, w.counters, 16, cudaMemcpyDeviceToHost, q), "counters");
-        if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "render");
-        rays_closest = cnt[0];
-        rays_shadow = cnt[1];
+        counted = true;
     }
     cudaEventRecord(ctx->ev1, q);
     if (st == MRT_OK) st = cuda_status(ctx, cudaGetLastError(), "render kernels");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaEventSynchronize(ctx->ev1), "render");
+    if (st == MRT_OK && counted)
+        st = cuda_status(ctx, cudaMemcpyAsync(ctx->status->count, ctx->ray_counters(), 16, cudaMemcpyDeviceToHost, q), "counters");
+    // one wait for everything: the event, the counters and the error flag are in host memory after it
     if (st == MRT_OK) st = check_kernel_error(ctx);
+    if (counted) {
+        rays_closest = ctx->status->count[0];
+        rays_shadow = ctx->status->count[1];
+    }
     s->progress.store(o->spp);
     add_trace_time();
     if (stats) {

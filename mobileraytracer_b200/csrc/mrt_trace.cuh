@@ -23,7 +23,7 @@ MRT_HD uint32_t hid(uint32_t type, uint32_t index) { return MRT_HIT_ID(type, ind
 
 template <class S>
 __device__ __forceinline__ void raise_error(const S &s, int code) {
-    if (s.error_flag) atomicMax(s.error_flag, code);
+    if (s.error_flag) *const_cast<volatile int32_t *>(s.error_flag) = code;   // host memory: a plain store
 }
 
 // the fields of a scene the FAST-BVH node and leaf steps read; a persistent lane that traces in a
