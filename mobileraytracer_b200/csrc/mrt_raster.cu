@@ -27,8 +27,8 @@
 //     (one 64-bit atomicMin of (depth bits, ~triangle index) per covered pixel);
 //   * the fragment colour is the triangle's colour (all three vertices carry it), converted to 8 bits
 //     by round(clamp(c, 0, 1) * 255).
-// One thread sets up and clips each triangle and covers the pixels of small ones (bounding box of at
-// most 64 pixels, the soups' case); larger ones go to a queue that a block per triangle covers.
+// One thread sets up and clips each triangle; a warp covers the pixels of its small ones (bounding box of at
+// most 64 pixels, the soups' case) together; larger ones go to a queue that a block per triangle covers.
 #include <algorithm>
 #include <cmath>
 
@@ -361,12 +361,43 @@ __device__ __noinline__ void draw_clipped(const RasterParams &p, uint32_t tri, C
     for (int k = 1; k + 1 < n; ++k) draw_sub(p, tri, setup_sub(p, w[0], w[k], w[k + 1]), qslot, drawn, frags);
 }
 
-// one thread per triangle of the pass: all scene triangles, or the overflow list of the last pass
-__global__ void __launch_bounds__(128, 8) k_raster_tris(DevScene s, RasterParams p, const uint32_t *list, uint32_t n_items) {
+// A small triangle whose corners lie within kTight of each other (64 pixels): every edge function at a pixel
+// centre of its box, and its area, fit 32 bits, with the values the 64-bit form has.
+constexpr int32_t kTight = 64 * 256;
+struct __align__(16) SmallTri {   // 64 bytes of shared memory
+    int32_t r0, r1, r2;           // edge functions at the centre of the box's first pixel
+    uint32_t start;               // its first pixel among the warp's
+    int32_t dx12, dy12, dx20, dy20;
+    int32_t dx01, dy01;
+    uint32_t x0y0;                // first pixel: x | y << 16
+    uint32_t width;               // box width | ceil(65536 / width) << 8 | top-left bits of the edges << 29
+    float z0, dz1, dz2, inv_area;
+};
+
+__device__ __forceinline__ int32_t edge_fn32(int32_t xa, int32_t ya, int32_t xb, int32_t yb, int32_t px, int32_t py) {
+    return (xb - xa) * (py - ya) - (yb - ya) * (px - xa);
+}
+
+// A thread sets up one triangle of the pass (all scene triangles, or the overflow list of the last pass);
+// then each warp covers the boxes of its 32 triangles together, 32 pixels at a time: half the triangles
+// face away and the others' boxes hold 1 to 64 pixels, so a thread per triangle left 10.8 of 32 lanes at
+// work (64-bit edge functions besides).  The counts are added up over the block: two atomics a warp on the
+// same two words were the kernel's tail.  A preview of the 1,000,000-triangle soup at 1920x1080 takes 120 us, 165 before.
+constexpr int kRasterThreads = 256;
+__global__ void __launch_bounds__(kRasterThreads) k_raster_tris(DevScene s, RasterParams p, const uint32_t *list, uint32_t n_items) {
+    __shared__ SmallTri s_tri[kRasterThreads];
+    __shared__ uint32_t s_id[kRasterThreads];
+    __shared__ unsigned long long s_count[2];
+    const uint32_t FULL = 0xFFFFFFFFu;
+    const int lane = threadIdx.x & 31, warp0 = threadIdx.x & ~31;
+    if (threadIdx.x < 2) s_count[threadIdx.x] = 0;
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     unsigned long long drawn = 0, frags = 0;
+    uint32_t n_px = 0, tri = 0;
+    SmallTri e;
     if (i < n_items) {
-        const uint32_t tri = list ? list[i] : i;
+        tri = list ? list[i] : i;
         const float4 a = s.tri_a[tri], ab = s.tri_ab[tri], ac = s.tri_ac[tri];
         // DrawView.cpp:131-154: A, A + AB, A + AC, z negated
         const Clip c0 = to_clip(p.m, a.x, a.y, -a.z);
@@ -376,19 +407,99 @@ __global__ void __launch_bounds__(128, 8) k_raster_tris(DevScene s, RasterParams
         for (int q = 0; q < 6; ++q)
             inside = inside && plane_dist(c0, q) >= 0.0f && plane_dist(c1, q) >= 0.0f && plane_dist(c2, q) >= 0.0f;
         if (inside) {
-            const SubTri u = setup_sub(p, to_window(p, c0), to_window(p, c1), to_window(p, c2));
-            uint32_t qslot = 0;
-            if (reserve(p, tri, u.kind == 2 ? 1u : 0u, qslot)) draw_sub(p, tri, u, qslot, drawn, frags);
+            const Win w0 = to_window(p, c0), w1 = to_window(p, c1), w2 = to_window(p, c2);
+            const int32_t xmin = min(w0.x, min(w1.x, w2.x)), xmax = max(w0.x, max(w1.x, w2.x));
+            const int32_t ymin = min(w0.y, min(w1.y, w2.y)), ymax = max(w0.y, max(w1.y, w2.y));
+            if ((long long)xmax - xmin <= kTight && (long long)ymax - ymin <= kTight) {
+                const int32_t area2 = edge_fn32(w0.x, w0.y, w1.x, w1.y, w2.x, w2.y);
+                if (area2 > 0) {   // else clockwise (back face, culled) or no area
+                    ++drawn;
+                    // the pixels whose centres lie in the box and the viewport (256 ths, rounded inwards)
+                    const int32_t bx0 = max(0, (xmin + 127) >> 8), bx1 = min((int32_t)p.width - 1, (xmax - 128) >> 8);
+                    const int32_t by0 = max(0, (ymin + 127) >> 8), by1 = min((int32_t)p.height - 1, (ymax - 128) >> 8);
+                    if (bx0 <= bx1 && by0 <= by1) {
+                        const uint32_t w = (uint32_t)(bx1 - bx0 + 1), h = (uint32_t)(by1 - by0 + 1);
+                        if (w * h > kSmallPixels) {
+                            uint32_t qslot = 0;
+                            if (reserve(p, tri, 1u, qslot)) draw_sub(p, tri, setup_sub(p, w0, w1, w2), qslot, drawn, frags);
+                            --drawn;   // counted by draw_sub, or by the pass the triangle was sent on to
+                        } else {
+                            const int32_t cx = bx0 * 256 + 128, cy = by0 * 256 + 128;
+                            e.r0 = edge_fn32(w1.x, w1.y, w2.x, w2.y, cx, cy);
+                            e.r1 = edge_fn32(w2.x, w2.y, w0.x, w0.y, cx, cy);
+                            e.r2 = edge_fn32(w0.x, w0.y, w1.x, w1.y, cx, cy);
+                            e.dx12 = w2.x - w1.x; e.dy12 = w2.y - w1.y;
+                            e.dx20 = w0.x - w2.x; e.dy20 = w0.y - w2.y;
+                            e.dx01 = w1.x - w0.x; e.dy01 = w1.y - w0.y;
+                            e.x0y0 = (uint32_t)bx0 | (uint32_t)by0 << 16;
+                            e.width = w | ((65535u + w) / w) << 8 | (top_left(w1.x, w1.y, w2.x, w2.y) ? 1u << 29 : 0u) |
+                                      (top_left(w2.x, w2.y, w0.x, w0.y) ? 1u << 30 : 0u) |
+                                      (top_left(w0.x, w0.y, w1.x, w1.y) ? 1u << 31 : 0u);
+                            e.z0 = w0.z; e.dz1 = w1.z - w0.z; e.dz2 = w2.z - w0.z;
+                            e.inv_area = 1.0f / (float)area2;
+                            n_px = w * h;
+                        }
+                    }
+                }
+            } else {
+                const SubTri u = setup_sub(p, w0, w1, w2);
+                uint32_t qslot = 0;
+                if (reserve(p, tri, u.kind == 2 ? 1u : 0u, qslot)) draw_sub(p, tri, u, qslot, drawn, frags);
+            }
         } else {
             draw_clipped(p, tri, c0, c1, c2, drawn, frags);
         }
     }
-    drawn = warp_sum(drawn);
-    frags = warp_sum(frags);
-    if ((threadIdx.x & 31) == 0) {
-        if (drawn) atomicAdd(&p.counts[1], (unsigned long long)drawn);
-        if (frags) atomicAdd(&p.counts[2], (unsigned long long)frags);
+    // the warp's boxes one after the other: the triangles that have one packed into its shared slots
+    __syncwarp();
+    uint32_t end = n_px;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t v = __shfl_up_sync(FULL, end, o);
+        if (lane >= o) end += v;
     }
+    const uint32_t start = end - n_px, total = __shfl_sync(FULL, end, 31);
+    const uint32_t have = __ballot_sync(FULL, n_px != 0u);
+    if (n_px) {
+        const int slot = warp0 + __popc(have & ((1u << lane) - 1u));
+        e.start = start;
+        s_tri[slot] = e;
+        s_id[slot] = tri;
+    }
+    __syncwarp();
+    uint32_t before = 0;   // triangles whose box starts in an earlier round
+    for (uint32_t base = 0; base < total; base += 32) {
+        // bit k: a box starts at pixel base + k
+        const uint32_t starts = __reduce_or_sync(FULL, n_px && start - base < 32u ? 1u << (start - base) : 0u);
+        const uint32_t px = base + lane;
+        if (px < total) {
+            const int slot = warp0 + (int)(before + __popc(starts & (0xFFFFFFFFu >> (31 - lane)))) - 1;
+            const SmallTri t = s_tri[slot];
+            const uint32_t local = px - t.start, w = t.width & 0xFFu;
+            const uint32_t y = (local * ((t.width >> 8) & 0x1FFFFu)) >> 16, x = local - y * w;   // local < 64, w <= 64
+            const int32_t fx = (int32_t)x * 256, fy = (int32_t)y * 256;
+            const int32_t w0 = t.r0 - fx * t.dy12 + fy * t.dx12;
+            const int32_t w1 = t.r1 - fx * t.dy20 + fy * t.dx20;
+            const int32_t w2 = t.r2 - fx * t.dy01 + fy * t.dx01;
+            if ((w0 > 0 || (w0 == 0 && (t.width & 1u << 29))) && (w1 > 0 || (w1 == 0 && (t.width & 1u << 30))) &&
+                (w2 > 0 || (w2 == 0 && (t.width & 1u << 31)))) {
+                float z = t.z0 + ((float)w1 * t.dz1 + (float)w2 * t.dz2) * t.inv_area;
+                if (!(z > 0.0f)) z = 0.0f;
+                if (z > 1.0f) z = 1.0f;
+                const uint32_t fx0 = (t.x0y0 & 0xFFFFu) + x, fy0 = (t.x0y0 >> 16) + y;
+                atomicMin(&p.keys[(size_t)fy0 * p.width + fx0], depth_key(z, s_id[slot]));
+                ++frags;
+            }
+        }
+        before += __popc(starts);
+    }
+    // (at most 32 lanes x 14 pieces x 64 pixels: the sums fit 32 bits)
+    const uint32_t d = __reduce_add_sync(FULL, (uint32_t)drawn), f = __reduce_add_sync(FULL, (uint32_t)frags);
+    if (lane == 0) {
+        if (d) atomicAdd(&s_count[0], (unsigned long long)d);
+        if (f) atomicAdd(&s_count[1], (unsigned long long)f);
+    }
+    __syncthreads();
+    if (threadIdx.x < 2 && s_count[threadIdx.x]) atomicAdd(&p.counts[1 + threadIdx.x], s_count[threadIdx.x]);
 }
 
 // the queued triangles: a block per triangle, its threads over the pixel box
@@ -514,7 +625,7 @@ extern "C" int mrt_raster_preview(MrtScene *s, const MrtCamera *cam, uint32_t wi
     cudaMemsetAsync(p.keys, 0xFF, 8 * pixels, q);
     cudaMemsetAsync(p.counts, 0, 4 * sizeof(unsigned long long), q);
     if (s->n_tri > 0) {
-        k_raster_tris<<<(s->n_tri + 127) / 128, 128, 0, q>>>(s->dev, p, nullptr, s->n_tri);
+        k_raster_tris<<<(s->n_tri + kRasterThreads - 1) / kRasterThreads, kRasterThreads, 0, q>>>(s->dev, p, nullptr, s->n_tri);
         k_raster_big<<<ctx->sm_count * 8, 256, 0, q>>>(p);
     }
     k_raster_resolve<<<grid, 256, 0, q>>>(s->dev, p, d_bitmap, stride_bytes / 4u);
@@ -534,7 +645,7 @@ extern "C" int mrt_raster_preview(MrtScene *s, const MrtCamera *cam, uint32_t wi
         p.overflow = in == lists[0] ? lists[1] : lists[0];
         cudaMemsetAsync(p.counts, 0, sizeof(unsigned long long), q);
         cudaMemsetAsync(p.counts + 3, 0, sizeof(unsigned long long), q);
-        k_raster_tris<<<(n_items + 127) / 128, 128, 0, q>>>(s->dev, p, in, n_items);
+        k_raster_tris<<<(n_items + kRasterThreads - 1) / kRasterThreads, kRasterThreads, 0, q>>>(s->dev, p, in, n_items);
         k_raster_big<<<ctx->sm_count * 8, 256, 0, q>>>(p);
         k_raster_resolve<<<grid, 256, 0, q>>>(s->dev, p, d_bitmap, stride_bytes / 4u);
         st = cuda_status(ctx, cudaGetLastError(), "raster kernels");
