@@ -262,14 +262,14 @@ __global__ void __launch_bounds__(128) k_ns_shade_visits(DevScene s, RenderParam
                                                          uint32_t n_first, uint32_t s0, uint32_t n_s,
                                                          const uint2 *__restrict__ hits) {
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_first; j += gridDim.x * blockDim.x) {
-        const uint32_t index = p.tasks[j].index;
-        uint32_t bm = p.bitmap[index];
-        const int64_t slot = p.accum ? accum_slot(p, p.tasks[j]) : -1;
+        const Task first = task_of(p, j);
+        uint32_t bm = p.bitmap[first.index];
+        const int64_t slot = p.accum ? accum_slot(p, first) : -1;
         float4 acc = slot >= 0 ? p.accum[slot] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         for (uint32_t si = 0; si < n_s; ++si) {
             const uint32_t sample = p.spp_offset + s0 + si;
             for (uint32_t t = j; t != kNoTask; t = next_visit[t]) {
-                const Task k = p.tasks[t];
+                const Task k = task_of(p, t);
                 const uint2 h = hits[(size_t)si * p.n_tasks + t];
                 V3 rgb{0.0f, 0.0f, 0.0f};
                 if (h.y != MRT_HIT_NONE) {
@@ -282,7 +282,7 @@ __global__ void __launch_bounds__(128) k_ns_shade_visits(DevScene s, RenderParam
                 acc.x += rgb.x; acc.y += rgb.y; acc.z += rgb.z; acc.w += 1.0f;
             }
         }
-        p.bitmap[index] = bm;
+        p.bitmap[first.index] = bm;
         if (slot >= 0) p.accum[slot] = acc;
     }
 }
@@ -630,7 +630,7 @@ struct TaskPlan {
     bool uploaded = false;               // explicit list already in the scene's work[0]
     bool implicit = true;
     uint32_t n_tasks = 0;
-    std::vector<Task> list;                  // explicit tasks by round
+    std::vector<uint2> list;                 // explicit tasks (x, y) by round
     std::vector<uint32_t> next_visit;        // the same pixel's task in the next round (kNoTask: none)
     std::vector<uint32_t> round_first, round_count;
 };
@@ -642,8 +642,15 @@ bool plan_tasks(const MrtRenderOpts &o, uint32_t stride_px, TaskPlan &plan) {
     if (bsx == 0 || bsy == 0) return false;
     const uint32_t domain = (w / bsx) * (h / bsy);
     const uint64_t res = (uint64_t)w * h;
-    std::vector<Task> tasks;
-    tasks.reserve((size_t)256 * bsx * bsy);
+    // Every visit of a pixel goes to the round of its number (a round renders a pixel at most once), block
+    // order kept per pixel; tasks outside the bitmap (undefined behaviour in the reference) are dropped.
+    const size_t n_px = (size_t)stride_px * h;
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    std::vector<std::vector<uint2>> rounds;      // by round and bitmap pixel (x = kNone: not rendered)
+    std::vector<uint32_t> round_size, visits(n_px, 0);
+    uint64_t n_all = 0;
+    bool inside = true;   // every task in the rectangle [0, w) x [0, rows)
+    const uint32_t rows = 16u * bsy;
     for (uint32_t i = 0; i < 256; ++i) {
         const float block = halton(i, 2);
         const uint32_t rb = (uint32_t)roundf(block * (float)domain);
@@ -652,58 +659,54 @@ bool plan_tasks(const MrtRenderOpts &o, uint32_t stride_px, TaskPlan &plan) {
         for (uint32_t y = sy; y < sy + bsy; ++y) {
             const uint32_t yw = y * stride_px;
             const uint32_t sx = (pixel + yw) % w;
-            for (uint32_t x = sx; x < sx + bsx; ++x) tasks.push_back(Task{x, y, yw + x});
+            n_all += bsx;
+            inside = inside && y < rows && sx + bsx <= w;
+            for (uint32_t x = sx; x < sx + bsx; ++x) {
+                const uint32_t index = yw + x;
+                if ((uint64_t)index >= (uint64_t)n_px) continue;
+                const uint32_t r = visits[index]++;
+                if (r >= rounds.size()) {
+                    rounds.emplace_back(n_px, make_uint2(kNone, 0u));
+                    round_size.push_back(0);
+                }
+                rounds[r][index] = make_uint2(x, y);
+                ++round_size[r];
+            }
         }
     }
     // the implicit rectangle?
-    const uint32_t rows = 16u * bsy;
-    bool rect = tasks.size() == (size_t)w * rows;
-    std::vector<uint8_t> seen((size_t)stride_px * h + 1, 0);
-    if (rect) {
-        for (const Task &t : tasks) {
-            if (t.x >= w || t.y >= rows || t.index != t.y * stride_px + t.x || seen[t.index]) { rect = false; break; }
-            seen[t.index] = 1;
-        }
-    }
-    if (rect) {
+    if (inside && n_all == (uint64_t)w * rows && rounds.size() == 1 && round_size[0] == n_all) {
         plan.implicit = true;
         plan.n_tasks = w * rows;
         plan.round_first = {0};
         plan.round_count = {plan.n_tasks};
         return true;
     }
-    // explicit: drop tasks outside the bitmap (undefined behaviour in the reference), then rounds
-    // in which every pixel appears at most once, preserving block order per pixel
     plan.implicit = false;
-    std::vector<uint32_t> visits((size_t)stride_px * h + 1, 0);
-    std::vector<std::vector<Task>> rounds;
-    for (const Task &t : tasks) {
-        if ((uint64_t)t.index >= (uint64_t)stride_px * h) continue;   // outside the bitmap
-        const uint32_t r = visits[t.index]++;
-        if (rounds.size() <= r) rounds.emplace_back();
-        rounds[r].push_back(t);
-    }
-    // a round renders a pixel once, so its order is free: 2x16-pixel tiles of the bitmap, one after the
-    // other, so that the 32 rays a warp takes are neighbours (in block order a warp takes a row of 32)
-    for (auto &r : rounds) {
+    // a round's order is free: 2x16-pixel tiles of the bitmap, one after the other, so that the 32 rays a
+    // warp takes are neighbours (in block order a warp takes a row of 32)
+    for (size_t k = 0; k < rounds.size(); ++k) {
+        std::vector<uint2> &at = rounds[k];
         plan.round_first.push_back((uint32_t)plan.list.size());
-        plan.round_count.push_back((uint32_t)r.size());
+        plan.round_count.push_back(round_size[k]);
         const uint32_t first = (uint32_t)plan.list.size();
-        std::vector<uint32_t> at((size_t)stride_px * h, kNoTask);
-        for (uint32_t i = 0; i < (uint32_t)r.size(); ++i) at[r[i].index] = i;
-        plan.list.reserve(plan.list.size() + r.size());
+        plan.list.reserve(plan.list.size() + round_size[k]);
         for (uint32_t y0 = 0; y0 < h; y0 += 16)
             for (uint32_t x0 = 0; x0 < stride_px; x0 += 2)
-                for (uint32_t y = y0; y < std::min(y0 + 16u, h); ++y)
+                for (uint32_t y = y0; y < std::min(y0 + 16u, h); ++y) {
+                    uint2 *row = &at[(size_t)y * stride_px];
                     for (uint32_t x = x0; x < std::min(x0 + 2u, stride_px); ++x) {
-                        uint32_t &i = at[(size_t)y * stride_px + x];
-                        if (i == kNoTask) continue;
-                        plan.list.push_back(r[i]);
-                        i = (uint32_t)plan.list.size() - 1u;   // from here on the task's place in the list
+                        if (row[x].x == kNone) continue;
+                        plan.list.push_back(row[x]);
+                        row[x].y = (uint32_t)plan.list.size() - 1u;   // from here on the task's place in the list
                     }
+                }
         // link the round before to this one
-        if (plan.round_first.size() > 1)
-            for (uint32_t t = plan.round_first[plan.round_first.size() - 2]; t < first; ++t) plan.next_visit[t] = at[plan.list[t].index];
+        if (k > 0)
+            for (uint32_t t = plan.round_first[k - 1]; t < first; ++t) {
+                const uint2 next = at[(size_t)plan.list[t].y * stride_px + plan.list[t].x];
+                plan.next_visit[t] = next.x == kNone ? kNoTask : next.y;
+            }
         plan.next_visit.resize(plan.list.size(), kNoTask);
     }
     plan.n_tasks = (uint32_t)plan.list.size();
@@ -824,17 +827,17 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
     int st = MRT_OK;
     if (!plan.implicit) {
         if (!plan.uploaded) {
-            st = ensure(ctx, s->work[0], (sizeof(Task) + sizeof(uint32_t)) * plan.list.size());
+            st = ensure(ctx, s->work[0], (sizeof(uint2) + sizeof(uint32_t)) * plan.list.size());
             if (st == MRT_OK)
-                st = cuda_status(ctx, cudaMemcpyAsync(s->work[0].ptr, plan.list.data(), sizeof(Task) * plan.list.size(),
+                st = cuda_status(ctx, cudaMemcpyAsync(s->work[0].ptr, plan.list.data(), sizeof(uint2) * plan.list.size(),
                                                       cudaMemcpyHostToDevice, q), "tasks");
             if (st == MRT_OK)
-                st = cuda_status(ctx, cudaMemcpyAsync((Task *)s->work[0].ptr + plan.list.size(), plan.next_visit.data(),
+                st = cuda_status(ctx, cudaMemcpyAsync((uint2 *)s->work[0].ptr + plan.list.size(), plan.next_visit.data(),
                                                       sizeof(uint32_t) * plan.list.size(), cudaMemcpyHostToDevice, q), "tasks");
             if (st != MRT_OK) return st;
             plan.uploaded = true;
         }
-        p.tasks = (const Task *)s->work[0].ptr;
+        p.tasks = (const uint2 *)s->work[0].ptr;
     }
     const int accel = s->opts.accelerator, mode = s->opts.bvh_mode;
     const bool fast = accel == MRT_ACCEL_BVH && mode == MRT_BVH_FAST;

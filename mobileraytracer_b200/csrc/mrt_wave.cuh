@@ -22,8 +22,8 @@ struct RenderParams {
     uint32_t spp_offset;
     uint32_t strata;       // spp of the whole render (Stratified sampler strata)
     uint32_t task_base;    // first task of the current round (wavefront)
-    // tasks: implicit rectangle (tasks == nullptr: x = t % width, y = t / width) or explicit list
-    const Task *tasks;
+    // tasks: implicit rectangle (tasks == nullptr: x = t % width, y = t / width) or explicit list of (x, y)
+    const uint2 *tasks;
     uint32_t n_tasks;
     uint32_t *bitmap;
     float4 *accum;
@@ -37,10 +37,15 @@ MRT_HD bool direct_shader(int shader) {
 }
 
 __device__ __forceinline__ Task task_of(const RenderParams &p, uint32_t t) {
-    if (p.tasks) return p.tasks[t];
     Task k;
-    k.x = t % p.width;
-    k.y = t / p.width;
+    if (p.tasks) {
+        const uint2 xy = p.tasks[t];
+        k.x = xy.x;
+        k.y = xy.y;
+    } else {
+        k.x = t % p.width;
+        k.y = t / p.width;
+    }
     k.index = k.y * p.stride_px + k.x;
     return k;
 }
