@@ -214,7 +214,7 @@ struct BatchPathWork {
     }
 };
 
-__global__ void __launch_bounds__(128, 8) k_batch_paths(BatchState b) {
+__global__ void __launch_bounds__(128, kPathBlocksPerSm) k_batch_paths(BatchState b) {
     BatchPathWork work{b, b.work};
     persistent_paths(work);
 }
@@ -471,7 +471,7 @@ void launch_trace_kernels(MrtBatch *b, int pipe, uint32_t threads, uint32_t bps,
     const int grid = sm * 16;
     if (threads == 0) {
         k_batch_begin<<<1, 64, 0, q>>>(s);
-        k_batch_paths<<<sm * 8, 128, 0, q>>>(s);
+        k_batch_paths<<<sm * kPathBlocksPerSm, 128, 0, q>>>(s);
         return;
     }
     auto trav = [&](int level, bool extend) {

@@ -22,6 +22,10 @@
 
 namespace mrt {
 
+// resident blocks of 128 threads per SM of the whole-path kernels (5: 94 registers without spills, the Cornell
+// Whitted frame 105.6 us; 4: 104.3, 8: 64 registers and 506 bytes of spills, 115; batches of 11 and 12 soups
+// 0.633 and 2.59 ms at 5, 0.643 and 2.66 at 4, 0.667 and 2.63 at 8)
+constexpr int kPathBlocksPerSm = 5;
 constexpr int kPathFrames = 12;   // recursion depth a lane can hold: depth_max + 1 <= kPathFrames
 
 struct PathFrame {

@@ -567,7 +567,7 @@ struct WavePathWork {
     }
 };
 
-__global__ void __launch_bounds__(128, 8) k_wave_paths(DevScene s, RenderParams p, WaveState w, uint32_t *ctr) {
+__global__ void __launch_bounds__(128, kPathBlocksPerSm) k_wave_paths(DevScene s, RenderParams p, WaveState w, uint32_t *ctr) {
     WavePathWork work{&s, &p, w, ctr};
     persistent_paths(work);
 }
@@ -1040,7 +1040,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
                 if (paths) {
                     if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
-                    k_wave_paths<<<ctx->sm_count * 8, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
+                    k_wave_paths<<<ctx->sm_count * kPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
                     launches += 2;   // with the fold below
                 } else {
                     cudaMemsetAsync(w.levels, 0, sizeof(Level) * (levels + 2), q);
