@@ -310,6 +310,8 @@ int mrt_context_create(int device, MrtContext **out) {
     for (auto &e : ctx->band_ev)
         if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking), "stream");
+    if (st == MRT_OK) st = cuda_status(ctx, cudaStreamCreateWithFlags(&ctx->wave_stream, cudaStreamNonBlocking), "stream");
+    if (st == MRT_OK) st = cuda_status(ctx, cudaEventCreateWithFlags(&ctx->fork_ev, cudaEventDisableTiming), "event");
 
     if (st != MRT_OK) {
         fprintf(stderr, "mrt_context_create: %s\n", ctx->error.c_str());
@@ -325,6 +327,7 @@ void mrt_context_destroy(MrtContext *ctx) {
     cudaSetDevice(ctx->device);
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
     if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
+    if (ctx->wave_stream) cudaStreamSynchronize(ctx->wave_stream);
     for (auto &b : ctx->scratch) dev_free(b);
     for (auto &b : ctx->wave) dev_free(b);
     for (auto &b : ctx->raster) dev_free(b);
@@ -336,7 +339,9 @@ void mrt_context_destroy(MrtContext *ctx) {
     for (auto &e : ctx->trace_ev) if (e) cudaEventDestroy(e);
     for (auto &e : ctx->wave_ev) if (e) cudaEventDestroy(e);
     for (auto &e : ctx->band_ev) if (e) cudaEventDestroy(e);
+    if (ctx->fork_ev) cudaEventDestroy(ctx->fork_ev);
     if (ctx->copy_stream) cudaStreamDestroy(ctx->copy_stream);
+    if (ctx->wave_stream) cudaStreamDestroy(ctx->wave_stream);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }

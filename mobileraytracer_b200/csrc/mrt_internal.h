@@ -49,15 +49,18 @@ struct MrtContext {
     };
     Status *status = nullptr;           // host address
     int32_t *d_error = nullptr;         // device address of status->error
-    // work counters of the persistent kernels (64 slots), then the two ray counters of a render
+    // work counters of the persistent kernels (64 for each wave in flight), then the two ray counters of a render
     uint32_t *d_counters = nullptr;
-    static constexpr int kWorkCounters = 64;
+    static constexpr int kWaveCounters = 64;       // of one wave
+    static constexpr int kWorkCounters = 2 * kWaveCounters;
     unsigned long long *ray_counters() const { return reinterpret_cast<unsigned long long *>(d_counters + kWorkCounters); }
     cudaMemPool_t pool = nullptr;       // the device's pool (mrt_capi.cu)
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     static constexpr int kTraceEvents = 16;             // start / end pairs around traversal launches
     cudaEvent_t trace_ev[2 * kTraceEvents] = {};
     cudaEvent_t wave_ev[2] = {nullptr, nullptr};   // the last two waves of a render (bounded run-ahead)
+    cudaStream_t wave_stream = nullptr;            // every other wave of a wavefront render
+    cudaEvent_t fork_ev = nullptr;
     static constexpr int kHostBands = 8;           // row bands a host-memory frame is shaded and copied out in
     cudaStream_t copy_stream = nullptr;            // device-to-host copies of finished bands
     cudaEvent_t band_ev[kHostBands] = {};

@@ -767,6 +767,7 @@ void launch_wave_level(const DevScene &s, const RenderParams &p, const WaveState
 // Renderer::stopRender seen between waves: the work already queued finishes (the caller's buffers
 // stay in use until then), the bitmap keeps the samples folded so far
 int cancelled(MrtContext *ctx, cudaStream_t q) {
+    cudaStreamSynchronize(ctx->wave_stream);
     cudaStreamSynchronize(q);
     set_error(ctx, "render stopped (mrt_render_stop)");
     return MRT_ERR_CANCELLED;
@@ -784,10 +785,18 @@ uint64_t paths_max_setting() {
     return v;
 }
 
+constexpr uint32_t kPairedRoots = 1u << 19;   // paths from which a wavefront runs as two waves at once
+
+// Paths in flight of a wavefront render: 2^22 where their queues (7 GB at depth 6) take at most an eighth of
+// the free device memory, 2^21 otherwise and on an arena, whose owner has sized it (MRT_WAVE_ROOTS: that
+// many).  Larger waves pay fewer tails and launches: the 1024x1024x16 terrain PathTracer takes 39.1 ms at
+// 2^20, 31.2 at 2^21, 27.3 at 2^22, 25.8 at 2^23 (14 GB, whose first allocation costs more than it gives).
+constexpr uint32_t kWaveRoots = 1u << 21;
 uint32_t wave_roots_setting() {
     static uint32_t v = [] {
         const char *e = getenv("MRT_WAVE_ROOTS");
-        const long x = e ? atol(e) : (1l << 21);
+        const long x = e ? atol(e) : 0l;
+        if (!e) return 0u;
         return (uint32_t)std::max(1024l, std::min(x, 1l << 25));
     }();
     return v;
@@ -996,33 +1005,66 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                            o->depth_max >= 0 && o->depth_max + 1 <= kPathFrames;
         uint64_t max_round = 0;
         for (uint32_t c : plan.round_count) max_round = std::max<uint64_t>(max_round, c);
-        const uint32_t wave = (uint32_t)std::min<uint64_t>(max_round * o->spp,
-                                                           paths ? std::max(wave_roots_setting(), 1u << 22)
-                                                                 : wave_roots_setting());
         const int levels = std::max(1, o->depth_max + 1);
-        const uint64_t ray_cap = paths ? 0 : (uint64_t)wave * (uint64_t)(levels + 2);
-        const uint64_t shadow_cap = paths ? 0 : (uint64_t)wave * std::max(1u, o->spl) * 2ull;
-        if (ray_cap > 0xFFFFFFF0ull) { set_error(ctx, "mrt_render: wave too large"); return MRT_ERR_ARG; }
-        if (2 * (levels + 1) > 64) { set_error(ctx, "mrt_render: depth_max above 30"); return MRT_ERR_ARG; }
-        if (!paths) {   // the wavefront's queues (whole-path launches keep their state per lane)
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[1], kRayBytes * ray_cap);
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], kNodeBytes * ray_cap);
-            if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], kShadowBytes * shadow_cap);
+        uint32_t roots = wave_roots_setting();
+        if (!roots) {
+            roots = kWaveRoots;
+            const uint64_t need = 2ull * kWaveRoots * ((uint64_t)(levels + 2) * (kRayBytes + kNodeBytes) + std::max(1u, o->spl) * 2ull * kShadowBytes);
+            if (!paths && !ctx->arena && max_round * o->spp > kWaveRoots) {
+                size_t free_bytes = 0, all_bytes = 0;
+                const bool held = ctx->wave[2].bytes >= 2ull * kWaveRoots * (uint64_t)(levels + 2) * kNodeBytes;   // allocated before
+                if (held || (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && need <= free_bytes / 8)) roots = 2u * kWaveRoots;
+            }
         }
-        if (st == MRT_OK) st = ensure(ctx, ctx->wave[4], sizeof(Level) * (levels + 2));
-        if (st == MRT_OK) st = ensure(ctx, ctx->wave[5], sizeof(float4) * wave);
+        // Wavefronts of at least kPairedRoots paths run as two waves of half the size at once, each on its
+        // own stream and half of the queues: the tail of one wave's level (its longest rays, then a launch)
+        // overlaps the other's bulk (terrain PathTracer 32.0 -> 31.1 ms, glass room 2.22 -> 2.0 to 2.19).
+        // The folds stay in wave order.
+        int pipes = 1;
+        uint32_t wave = 0;
+        uint64_t ray_cap = 0, shadow_cap = 0;
+        for (;;) {
+            const uint32_t most = (uint32_t)std::min<uint64_t>(max_round * o->spp, paths ? std::max(roots, 1u << 22) : roots);
+            pipes = !paths && most >= kPairedRoots ? 2 : 1;
+            wave = (most + (uint32_t)pipes - 1u) / (uint32_t)pipes;
+            // (multiples of 4: the second wave's records start on 32 bytes)
+            ray_cap = paths ? 0 : ((uint64_t)wave * (uint64_t)(levels + 2) + 3) & ~3ull;
+            shadow_cap = paths ? 0 : ((uint64_t)wave * std::max(1u, o->spl) * 2ull + 3) & ~3ull;
+            if (ray_cap * pipes > 0xFFFFFFF0ull) { set_error(ctx, "mrt_render: wave too large"); return MRT_ERR_ARG; }
+            if (2 * (levels + 1) > MrtContext::kWaveCounters) { set_error(ctx, "mrt_render: depth_max above 30"); return MRT_ERR_ARG; }
+            if (!paths) {   // the wavefront's queues (whole-path launches keep their state per lane)
+                st = ensure(ctx, ctx->wave[1], kRayBytes * ray_cap * pipes);
+                if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], kNodeBytes * ray_cap * pipes);
+                if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], kShadowBytes * shadow_cap * pipes);
+            }
+            if (st != MRT_ERR_OOM || roots <= kWaveRoots) break;
+            roots = kWaveRoots;   // no room for the large wave after all
+            for (int k = 1; k <= 3; ++k) dev_free(ctx->wave[k]);
+            st = MRT_OK;
+        }
+        if (st == MRT_OK) st = ensure(ctx, ctx->wave[4], sizeof(Level) * (levels + 2) * pipes);
+        if (st == MRT_OK) st = ensure(ctx, ctx->wave[5], sizeof(float4) * (size_t)wave * pipes);
         if (st != MRT_OK) return st;
-        WaveState w{};
-        w.rec = wave_records(ctx->wave[1].ptr, ctx->wave[2].ptr, ctx->wave[3].ptr, (uint32_t)ray_cap, (uint32_t)shadow_cap);
-        w.levels = (Level *)ctx->wave[4].ptr;
-        w.root_rgb = (float4 *)ctx->wave[5].ptr;
-        w.counters = ctx->ray_counters();
-        // per-material shade queues where the scene mixes diffuse with mirror / glass materials
-        w.sort_shading = (o->flags & MRT_RENDER_SHADE_QUEUES) && s->mixed_materials ? 1u : 0u;
-        // the work counters of the first wave and the ray counters
+        WaveState pipe[2] = {};
+        for (int k = 0; k < pipes; ++k) {
+            WaveState &w = pipe[k];
+            if (!paths)
+                w.rec = wave_records((char *)ctx->wave[1].ptr + kRayBytes * ray_cap * k, (char *)ctx->wave[2].ptr + kNodeBytes * ray_cap * k,
+                                     (char *)ctx->wave[3].ptr + kShadowBytes * shadow_cap * k, (uint32_t)ray_cap, (uint32_t)shadow_cap);
+            w.levels = (Level *)ctx->wave[4].ptr + (levels + 2) * k;
+            w.root_rgb = (float4 *)ctx->wave[5].ptr + (size_t)wave * k;
+            w.counters = ctx->ray_counters();
+            // per-material shade queues where the scene mixes diffuse with mirror / glass materials
+            w.sort_shading = (o->flags & MRT_RENDER_SHADE_QUEUES) && s->mixed_materials ? 1u : 0u;
+        }
+        // the work counters of the first waves and the ray counters
         cudaMemsetAsync(ctx->d_counters, 0, MrtContext::kWorkCounters * sizeof(uint32_t) + 16, q);
-        // at most one wave queued ahead of the one running: a stop request ends the render within two
-        // waves, and progress counts finished waves
+        if (pipes == 2) {
+            cudaEventRecord(ctx->fork_ev, q);
+            cudaStreamWaitEvent(ctx->wave_stream, ctx->fork_ev, 0);
+        }
+        // at most two waves running or queued: a stop request ends the render within two waves, and
+        // progress counts finished waves
         uint64_t waves_issued = 0;
         uint64_t done_samples[2] = {0, 0};
         for (size_t rd = 0; rd < plan.round_first.size(); ++rd) {
@@ -1036,6 +1078,10 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                     s->progress.store((uint32_t)done_samples[slot]);
                 }
                 if (s->stop.load()) return cancelled(ctx, q);
+                const int k = pipes == 2 ? (int)(waves_issued % 2) : 0;
+                WaveState &w = pipe[k];
+                cudaStream_t wq = k ? ctx->wave_stream : q;
+                uint32_t *work = ctx->d_counters + k * MrtContext::kWaveCounters;
                 w.root_first = (uint32_t)r0;
                 w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
                 if (paths) {
@@ -1043,22 +1089,25 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                     k_wave_paths<<<ctx->sm_count * kPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
                     launches += 2;   // with the fold below
                 } else {
-                    cudaMemsetAsync(w.levels, 0, sizeof(Level) * (levels + 2), q);
-                    if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t) * 2 * (levels + 1), q);
-                    k_wave_raygen<<<grid, 128, 0, q>>>(p, w);
+                    cudaMemsetAsync(w.levels, 0, sizeof(Level) * (levels + 2), wq);
+                    if (waves_issued >= (uint64_t)pipes) cudaMemsetAsync(work, 0, sizeof(uint32_t) * 2 * (levels + 1), wq);
+                    k_wave_raygen<<<grid, 128, 0, wq>>>(p, w);
                     for (int b = 0; b < levels; ++b)
-                        MRT_DISPATCH(launch_wave_level, accel, mode, s->dev, p, w, b, grid, q, ctx->d_counters);
-                    for (int b = levels - 1; b >= 0; --b) k_wave_resolve<<<grid, 128, 0, q>>>(s->dev, p, w, b);
+                        MRT_DISPATCH(launch_wave_level, accel, mode, s->dev, p, w, b, grid, wq, work);
+                    for (int b = levels - 1; b >= 0; --b) k_wave_resolve<<<grid, 128, 0, wq>>>(s->dev, p, w, b);
                     launches += 2u + 4u * (uint32_t)levels;   // raygen, per level extend / shade / shadow /
                                                               // resolve, the fold below
                 }
-                k_wave_accumulate<<<grid, 128, 0, q>>>(p, w);
                 const int slot = (int)(waves_issued % 2);
-                cudaEventRecord(ctx->wave_ev[slot], q);
+                // a pixel's samples can straddle two waves: their folds run in wave order
+                if (pipes == 2 && waves_issued) cudaStreamWaitEvent(wq, ctx->wave_ev[1 - slot], 0);
+                k_wave_accumulate<<<grid, 128, 0, wq>>>(p, w);
+                cudaEventRecord(ctx->wave_ev[slot], wq);
                 done_samples[slot] = (r0 + w.n_roots) / std::max<uint64_t>(1, plan.round_count[rd]);
                 ++waves_issued;
             }
         }
+        if (pipes == 2 && waves_issued) cudaStreamWaitEvent(q, ctx->wave_ev[(waves_issued - 1) % 2], 0);
         counted = true;
     }
     cudaEventRecord(ctx->ev1, q);
