@@ -466,159 +466,176 @@ __device__ __forceinline__ int grid_exponent(float lo, float hi) {
     const double m = frexp(want, &ex);   // want = m 2^ex, m in [0.5, 1)
     return m == 0.5 ? ex - 1 : ex;
 }
-// a child's planes on the grid, lo rounded down and hi up (with a 2^-20 step guard against the
-// rounding of the double-precision subtraction), as lo | hi << 16
-__device__ __forceinline__ uint32_t quantise(float p, double step, float lo, float hi) {
-    double ql = floor(((double)lo - (double)p) / step - 0x1p-20);
-    double qh = ceil(((double)hi - (double)p) / step + 0x1p-20);
+// a child's planes on the grid of step 1 / inv_step (a power of two), lo rounded down and hi up (with a
+// 2^-20 step guard against the rounding of the double-precision subtraction), as lo | hi << 16
+__device__ __forceinline__ uint32_t quantise(float p, double inv_step, float lo, float hi) {
+    double ql = floor(((double)lo - (double)p) * inv_step - 0x1p-20);
+    double qh = ceil(((double)hi - (double)p) * inv_step + 0x1p-20);
     ql = fmin(fmax(ql, 0.0), 65535.0);
     qh = fmin(fmax(qh, 0.0), 65535.0);
     return (uint32_t)ql | ((uint32_t)qh << 16);
 }
 
-__device__ void collapse_node(const BinTree &t, CollapseItem it, int level, CollapseItem *out, uint32_t cap, uint4 *nodes,
-                              const float4 *__restrict__ a4, const float4 *__restrict__ ab4,
-                              const float4 *__restrict__ ac4, float4 *tris, uint32_t *ctrs) {
-    const uint32_t n_tri = t.n;
-    if (it.node >= cap) { atomicMax(&ctrs[1], 1u); return; }
-    uint32_t child[kWide];
-    int m = 0;
-    if (t.is_leaf(it.bin)) {   // only the root of a scene of at most kMaxLeafTris triangles
-        child[m++] = it.bin;
-    } else {
-        uint32_t st_node[kWide], st_slots[kWide];
-        int sp = 0;
-        const uint32_t k8 = choice_node_split(t.costs[it.bin].choice);
-        st_node[sp] = t.right[it.bin]; st_slots[sp++] = 8u - k8;
-        st_node[sp] = t.left[it.bin]; st_slots[sp++] = k8;
-        while (sp > 0) {
-            const uint32_t c = st_node[--sp];
-            uint32_t j = min(st_slots[sp], 7u), k = 0;
-            if (!(c & kLeafBit)) {
-                const uint32_t choice = t.costs[c].choice;
-                while (j > 1u && (k = choice_split(choice, j)) == 0u) --j;
-            }
-            if (k == 0u) {   // one slot
-                if (m >= kWide) { atomicMax(&ctrs[1], 1u); return; }
-                child[m++] = c;
-                continue;
-            }
-            if (sp + 2 > kWide) { atomicMax(&ctrs[1], 1u); return; }
-            st_node[sp] = t.right[c]; st_slots[sp++] = j - k;
-            st_node[sp] = t.left[c]; st_slots[sp++] = k;
-        }
-    }
-    float4 lo[kWide], hi[kWide];
-    bool internal[kWide];
-    float4 nlo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f), nhi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
-    for (int k = 0; k < m; ++k) {
-        const uint32_t c = child[k];
-        if (c & kLeafBit) {
-            const uint32_t tri = t.vals[c & ~kLeafBit];
-            lo[k] = t.bmin[tri];
-            hi[k] = t.bmax[tri];
-        } else {
-            lo[k] = t.imin[c];
-            hi[k] = t.imax[c];
-        }
-        internal[k] = !t.is_leaf(c);
-        nlo = make_float4(fminf(nlo.x, lo[k].x), fminf(nlo.y, lo[k].y), fminf(nlo.z, lo[k].z), 0.0f);
-        nhi = make_float4(fmaxf(nhi.x, hi[k].x), fmaxf(nhi.y, hi[k].y), fmaxf(nhi.z, hi[k].z), 0.0f);
-    }
-    // slots by octant: the child whose centre lies on the high side of axis a prefers slots with bit a set
-    const float cx = 0.5f * (nlo.x + nhi.x), cy = 0.5f * (nlo.y + nhi.y), cz = 0.5f * (nlo.z + nhi.z);
-    int slot_of[kWide];
-    uint32_t used = 0, placed = 0;
-    for (int k = 0; k < m; ++k) slot_of[k] = -1;
-    for (int round = 0; round < m; ++round) {
-        float best = 3.0e38f;
-        int bk = -1, bs = -1;
-        for (int k = 0; k < m; ++k) {
-            if ((placed >> k) & 1u) continue;
-            const float dx = 0.5f * (lo[k].x + hi[k].x) - cx, dy = 0.5f * (lo[k].y + hi[k].y) - cy,
-                        dz = 0.5f * (lo[k].z + hi[k].z) - cz;
-            for (int sl = 0; sl < kWide; ++sl) {
-                if ((used >> sl) & 1u) continue;
-                const float c = ((sl & 1) ? -dx : dx) + ((sl & 2) ? -dy : dy) + ((sl & 4) ? -dz : dz);
-                if (c < best) { best = c; bk = k; bs = sl; }
-            }
-        }
-        if (bk < 0) {   // non-finite centres: the first free slot
-            bk = __ffs(~placed & ((1u << m) - 1u)) - 1;
-            bs = __ffs(~used & 0xFFu) - 1;
-        }
-        slot_of[bk] = bs;
-        placed |= 1u << bk;
-        used |= 1u << bs;
-    }
-    int child_at[kWide];
-    for (int sl = 0; sl < kWide; ++sl) child_at[sl] = -1;
-    uint32_t imask = 0, n_int = 0, n_lt = 0;
-    for (int k = 0; k < m; ++k) {
-        child_at[slot_of[k]] = k;
-        if (internal[k]) { imask |= 1u << slot_of[k]; ++n_int; }
-        else n_lt += (child[k] & kLeafBit) ? 1u : t.last[child[k]] - t.first[child[k]] + 1u;
-    }
-    const uint32_t child_base = n_int ? atomicAdd(&ctrs[0], n_int) : 0u;
-    const uint32_t qpos = n_int ? atomicAdd(&ctrs[kLevelCtr + level + 1], n_int) : 0u;
-    const uint32_t tri_base = n_lt ? atomicAdd(&ctrs[2], n_lt) : 0u;
-    if ((uint64_t)child_base + n_int > cap || (uint64_t)qpos + n_int > cap || (uint64_t)tri_base + n_lt > n_tri) {
-        atomicMax(&ctrs[1], 1u);
-        return;
-    }
-    const int ex = grid_exponent(nlo.x, nhi.x), ey = grid_exponent(nlo.y, nhi.y), ez = grid_exponent(nlo.z, nhi.z);
-    if (ex > 127 || ey > 127 || ez > 127) { atomicMax(&ctrs[1], 2u); return; }
-    const double sx = ldexp(1.0, ex), sy = ldexp(1.0, ey), sz = ldexp(1.0, ez);
-    uint32_t w[kNodeWords];
-    w[0] = __float_as_uint(nlo.x);
-    w[1] = __float_as_uint(nlo.y);
-    w[2] = __float_as_uint(nlo.z);
-    w[3] = (uint32_t)(ex + 127) | ((uint32_t)(ey + 127) << 8) | ((uint32_t)(ez + 127) << 16) | (imask << 24);
-    w[kNodeChildBase] = child_base;
-    w[kNodeTriBase] = tri_base;
-    w[kNodeMeta] = w[kNodeMeta + 1] = 0;
-    uint32_t offset = 0, rank = 0;
-    for (int sl = 0; sl < kWide; ++sl) {
-        const int k = child_at[sl];
-        if (k < 0) {   // empty slot: an inverted box, no meta
-            w[node_plane_word(0, sl)] = w[node_plane_word(1, sl)] = w[node_plane_word(2, sl)] = 0xFFFFu;
-            continue;
-        }
-        w[node_plane_word(0, sl)] = quantise(nlo.x, sx, lo[k].x, hi[k].x);
-        w[node_plane_word(1, sl)] = quantise(nlo.y, sy, lo[k].y, hi[k].y);
-        w[node_plane_word(2, sl)] = quantise(nlo.z, sz, lo[k].z, hi[k].z);
-        if ((imask >> sl) & 1u) {
-            out[qpos + rank] = CollapseItem{child[k], child_base + rank};
-            ++rank;
-        } else {
-            const uint32_t c = child[k];
-            const uint32_t first = (c & kLeafBit) ? c & ~kLeafBit : t.first[c];
-            const uint32_t count = (c & kLeafBit) ? 1u : t.last[c] - first + 1u;
-            if (count == 0 || count > kMaxLeafTris || (uint64_t)first + count > n_tri) { atomicMax(&ctrs[1], 1u); return; }
-            w[kNodeMeta + (sl >> 2)] |= ((((1u << count) - 1u) << 5) | offset) << (8 * (sl & 3));
-            for (uint32_t j = 0; j < count; ++j) {
-                const uint32_t tri = t.vals[first + j];
-                const float4 a = a4[tri];
-                float4 *rec = tris + 3 * (size_t)(tri_base + offset + j);
-                rec[0] = make_float4(a.x, a.y, a.z, __uint_as_float(tri));
-                rec[1] = ab4[tri];
-                rec[2] = ac4[tri];
-            }
-            offset += count;
-        }
-    }
-    uint4 *dst = nodes + (size_t)it.node * (kNodeWords / 4);
-    for (int q = 0; q < kNodeWords / 4; ++q) dst[q] = make_uint4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
-}
-
-__global__ void __launch_bounds__(128) k_collapse(BinTree t, const CollapseItem *__restrict__ in, int level, CollapseItem *out,
-                                                  uint32_t cap, uint4 *nodes, const float4 *__restrict__ a4,
-                                                  const float4 *__restrict__ ab4, const float4 *__restrict__ ac4,
-                                                  float4 *tris, uint32_t *ctrs) {
+// Eight lanes make one wide node, a lane per child.  (One thread per node, its 512 slot
+// comparisons and 48 double-precision divisions in a row, took 20 to 30 us a level however few its nodes; a
+// 200,003-triangle scene opened and rendered once took 2.58 ms, 2.32 now.)
+constexpr int kCollapseThreads = 128, kGroups = kCollapseThreads / kWide;
+__global__ void __launch_bounds__(kCollapseThreads) k_collapse(BinTree t, const CollapseItem *__restrict__ in, int level,
+                                                               CollapseItem *out, uint32_t cap, uint32_t *nodes,
+                                                               const float4 *__restrict__ a4, const float4 *__restrict__ ab4,
+                                                               const float4 *__restrict__ ac4, float4 *tris, uint32_t *ctrs) {
     if (ctrs[1]) return;   // after an error the level's items may be unwritten
     const uint32_t n_in = min(ctrs[kLevelCtr + level], cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n_in; i += gridDim.x * blockDim.x)
-        collapse_node(t, in[i], level, out, cap, nodes, a4, ab4, ac4, tris, ctrs);
+    const int lane = threadIdx.x & (kWide - 1), group = threadIdx.x / kWide;
+    const int lane0 = threadIdx.x & 31 & ~(kWide - 1);       // the group's first lane in its warp
+    const uint32_t mask = 0xFFu << lane0;
+    auto from = [&](auto v, int k) { return __shfl_sync(mask, v, lane0 + k); };
+    for (uint32_t i = blockIdx.x * kGroups + group; i < n_in; i += gridDim.x * kGroups) {
+        const CollapseItem it = in[i];
+        // 1. the children: the binary node's two children in 8 slots, split on along the choices, all lanes'
+        // subtrees a step at a time (the chain of loads is as long as the deepest split, not as their number)
+        if (it.node >= cap) { if (lane == 0) atomicMax(&ctrs[1], 1u); continue; }
+        uint32_t c = it.bin, slots = 0, m = 1;
+        bool split = false;                       // the lane's subtree may have to be split further
+        if (!t.is_leaf(it.bin)) {                 // (else the root of a scene of at most kMaxLeafTris triangles)
+            const uint32_t k8 = choice_node_split(t.costs[it.bin].choice);
+            c = lane == 0 ? t.left[it.bin] : t.right[it.bin];
+            slots = lane == 0 ? k8 : 8u - k8;
+            m = 2;
+            split = lane < 2;
+        }
+        while (__any_sync(mask, split)) {
+            uint32_t k = 0, right = 0, right_slots = 0;
+            if (split && !(c & kLeafBit)) {
+                const uint32_t choice = t.costs[c].choice;
+                uint32_t j = min(slots, 7u);
+                while (j > 1u && (k = choice_split(choice, j)) == 0u) --j;
+                if (k) {
+                    right = t.right[c];
+                    right_slots = j - k;
+                    c = t.left[c];
+                    slots = k;
+                }
+            }
+            // the right halves go to the next free lanes (the slots add up to at most 8, so there are enough)
+            const uint32_t splitting = (__ballot_sync(mask, k != 0u) >> lane0) & 0xFFu;
+            const int mine = lane - (int)m;        // a free lane takes the half of the mine-th splitting lane
+            const int n_split = __popc(splitting);
+            uint32_t rest = splitting;
+            for (int q = 0; q < mine; ++q) rest &= rest - 1u;
+            const bool take = mine >= 0 && mine < n_split;
+            const int src = take ? __ffs(rest) - 1 : lane;
+            const uint32_t c_in = __shfl_sync(mask, right, lane0 + src), s_in = __shfl_sync(mask, right_slots, lane0 + src);
+            split = k != 0u;
+            if (take) { c = c_in; slots = s_in; split = true; }
+            m += (uint32_t)n_split;
+        }
+        if (m > (uint32_t)kWide) { if (lane == 0) atomicMax(&ctrs[1], 1u); continue; }
+        // 2. a lane's child: its box, and the node's
+        const bool have = lane < (int)m;
+        float4 lo = make_float4(3.0e38f, 3.0e38f, 3.0e38f, 0.0f), hi = make_float4(-3.0e38f, -3.0e38f, -3.0e38f, 0.0f);
+        bool internal = false;
+        uint32_t first = 0, count = 0;
+        if (have) {
+            if (c & kLeafBit) {
+                first = c & ~kLeafBit;
+                count = 1;
+                const uint32_t tri = t.vals[first];
+                lo = t.bmin[tri];
+                hi = t.bmax[tri];
+            } else {
+                lo = t.imin[c];
+                hi = t.imax[c];
+                internal = !t.is_leaf(c);
+                if (!internal) {
+                    first = t.first[c];
+                    count = t.last[c] - first + 1u;
+                }
+            }
+        }
+        float nlx = lo.x, nly = lo.y, nlz = lo.z, nhx = hi.x, nhy = hi.y, nhz = hi.z;
+        for (int o = 1; o < kWide; o <<= 1) {
+            nlx = fminf(nlx, __shfl_xor_sync(mask, nlx, o)); nly = fminf(nly, __shfl_xor_sync(mask, nly, o));
+            nlz = fminf(nlz, __shfl_xor_sync(mask, nlz, o)); nhx = fmaxf(nhx, __shfl_xor_sync(mask, nhx, o));
+            nhy = fmaxf(nhy, __shfl_xor_sync(mask, nhy, o)); nhz = fmaxf(nhz, __shfl_xor_sync(mask, nhz, o));
+        }
+        // 3. slots by octant: the child whose centre lies on the high side of axis a prefers slots with bit a
+        // set; the best (child, slot) of those left is placed, m times
+        const float dx = 0.5f * (lo.x + hi.x) - 0.5f * (nlx + nhx), dy = 0.5f * (lo.y + hi.y) - 0.5f * (nly + nhy),
+                    dz = 0.5f * (lo.z + hi.z) - 0.5f * (nlz + nhz);
+        uint32_t used = 0;
+        int slot = -1;
+        for (uint32_t round = 0; round < m; ++round) {
+            float best = 3.0e38f;
+            int bs = -1, bk = kWide;
+            if (have && slot < 0)
+                for (int sl = 0; sl < kWide; ++sl) {
+                    if ((used >> sl) & 1u) continue;
+                    const float v = ((sl & 1) ? -dx : dx) + ((sl & 2) ? -dy : dy) + ((sl & 4) ? -dz : dz);
+                    if (v < best || bs < 0) { best = v < best ? v : best; bs = sl; bk = lane; }   // (a free slot whatever v)
+                }
+            for (int o = 1; o < kWide; o <<= 1) {
+                const float v = __shfl_xor_sync(mask, best, o);
+                const int k = __shfl_xor_sync(mask, bk, o), sl = __shfl_xor_sync(mask, bs, o);
+                if (k < kWide && (bk == kWide || v < best || (v == best && k < bk))) { best = v; bk = k; bs = sl; }
+            }
+            if (lane == bk) slot = bs;
+            used |= 1u << bs;
+        }
+        // the lanes without a child take the free slots (their planes are an inverted box, their meta byte 0)
+        {
+            uint32_t rest = ~used & 0xFFu;
+            for (int k = (int)m; k < lane; ++k) rest &= rest - 1u;
+            if (!have) slot = __ffs(rest) - 1;
+        }
+        // 4. places: internal children in slot order, the leaf children's triangles in slot order
+        const uint32_t imask = __reduce_or_sync(mask, internal ? 1u << slot : 0u);
+        const uint32_t n_int = (uint32_t)__popc(imask), n_lt = __reduce_add_sync(mask, count);
+        uint32_t offset = 0;
+        for (int k = 0; k < kWide; ++k) {
+            const uint32_t ck = from(count, k);
+            if (from(slot, k) < slot) offset += ck;
+        }
+        uint32_t child_base = 0, qpos = 0, tri_base = 0;
+        if (lane == 0) {
+            if (n_int) child_base = atomicAdd(&ctrs[0], n_int);
+            if (n_int) qpos = atomicAdd(&ctrs[kLevelCtr + level + 1], n_int);
+            if (n_lt) tri_base = atomicAdd(&ctrs[2], n_lt);
+        }
+        child_base = from(child_base, 0);
+        qpos = from(qpos, 0);
+        tri_base = from(tri_base, 0);
+        const bool leaf_ok = !have || internal || (count > 0 && count <= kMaxLeafTris && (uint64_t)first + count <= t.n);
+        const int ex = grid_exponent(nlx, nhx), ey = grid_exponent(nly, nhy), ez = grid_exponent(nlz, nhz);
+        const uint32_t error = ((uint64_t)child_base + n_int > cap || (uint64_t)qpos + n_int > cap || (uint64_t)tri_base + n_lt > t.n ||
+                                !__all_sync(mask, leaf_ok)) ? 1u : ex > 127 || ey > 127 || ez > 127 ? 2u : 0u;
+        if (error) { if (lane == 0) atomicMax(&ctrs[1], error); continue; }
+        // 5. the node's words, the next level's items, the triangle records
+        uint32_t *w = nodes + (size_t)it.node * kNodeWords;
+        if (lane == 0) {
+            *reinterpret_cast<uint4 *>(w) = make_uint4(__float_as_uint(nlx), __float_as_uint(nly), __float_as_uint(nlz),
+                                                       (uint32_t)(ex + 127) | ((uint32_t)(ey + 127) << 8) |
+                                                           ((uint32_t)(ez + 127) << 16) | (imask << 24));
+            w[kNodeChildBase] = child_base;
+            w[kNodeTriBase] = tri_base;
+        }
+        w[node_plane_word(0, slot)] = have ? quantise(nlx, ldexp(1.0, -ex), lo.x, hi.x) : 0xFFFFu;
+        w[node_plane_word(1, slot)] = have ? quantise(nly, ldexp(1.0, -ey), lo.y, hi.y) : 0xFFFFu;
+        w[node_plane_word(2, slot)] = have ? quantise(nlz, ldexp(1.0, -ez), lo.z, hi.z) : 0xFFFFu;
+        reinterpret_cast<uint8_t *>(w + kNodeMeta)[slot] = count ? (uint8_t)((((1u << count) - 1u) << 5) | offset) : (uint8_t)0;
+        if (internal) {
+            const uint32_t rank = (uint32_t)__popc(imask & ((1u << slot) - 1u));
+            out[qpos + rank] = CollapseItem{c, child_base + rank};
+        }
+        for (uint32_t j = 0; j < count; ++j) {
+            const uint32_t tri = t.vals[first + j];
+            const float4 a = a4[tri];
+            float4 *rec = tris + 3 * (size_t)(tri_base + offset + j);
+            rec[0] = make_float4(a.x, a.y, a.z, __uint_as_float(tri));
+            rec[1] = ab4[tri];
+            rec[2] = ac4[tri];
+        }
+    }
 }
 
 }  // namespace
@@ -723,9 +740,9 @@ int build_fast_bvh(MrtScene *s) {
         for (const int stop = level + (level == 0 ? 10 : 4); level < stop; ++level) {
             if (level + 1 > kMaxLevels) { st = MRT_ERR_LIMIT; break; }
             const uint64_t most = level < 9 ? std::min<uint64_t>(1ull << (3 * level), cap) : cap;   // items of a level
-            const uint32_t blocks = (uint32_t)std::min<uint64_t>((most + 127) / 128, (uint64_t)ctx->sm_count * 16);
-            k_collapse<<<blocks, 128, 0, q>>>(bt, (const CollapseItem *)queue[level & 1].ptr, level,
-                                              (CollapseItem *)queue[1 - (level & 1)].ptr, cap, (uint4 *)wide.ptr,
+            const uint32_t blocks = (uint32_t)std::min<uint64_t>((most + kGroups - 1) / kGroups, (uint64_t)ctx->sm_count * 16);
+            k_collapse<<<blocks, kCollapseThreads, 0, q>>>(bt, (const CollapseItem *)queue[level & 1].ptr, level,
+                                              (CollapseItem *)queue[1 - (level & 1)].ptr, cap, (uint32_t *)wide.ptr,
                                               s->dev.tri_a, s->dev.tri_ab, s->dev.tri_ac, (float4 *)s->ftris.ptr,
                                               (uint32_t *)wctr.ptr);
         }
