@@ -326,8 +326,8 @@ __global__ void __launch_bounds__(128) k_wave_extend(DevScene s, WaveState w, in
     if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(&w.counters[0], (unsigned long long)L.count);
 }
 
-// one ray of a level shaded; every lane of the warp calls this (the child and shadow queues are
-// allocated once per warp)
+// one ray of a level shaded; every thread of the block calls this (places in the child and shadow queues
+// are allocated once per block)
 __device__ __forceinline__ void shade_slot(const DevScene &s, const RenderParams &p, const WaveState &w, int level,
                                            Level *next, uint32_t next_start, bool active, uint32_t idx) {
     ShadeLane o;
@@ -347,12 +347,10 @@ __device__ __forceinline__ void shade_slot(const DevScene &s, const RenderParams
         shade_ray(s, p, rr, hit.y, bitsf(hit.x), st, o);
         store_node(w.rec, idx, o.nd);
     }
-    // queue compaction: one atomic per warp for children, one for shadow rays
-    const uint32_t cbase = warp_alloc(o.n_child, &next->count);
-    const uint32_t sbase = warp_alloc(o.n_shadow, &w.levels[level].shadow_count);
+    const QueueSlots q = queue_slots(o, rr, st, &next->count, &w.levels[level].shadow_count);
     if (!active) return;
-    emit_children(s, o, rr, st, idx, next_start + cbase, w.rec);
-    emit_shadows(s, p, st, o, rr, idx, sbase, w.rec);
+    emit_children(s, o, rr, st, idx, next_start + q.child, w.rec, &q.first);
+    emit_shadows(s, p, st, o, rr, idx, q.shadow, w.rec);
 }
 
 // (8 blocks per SM: glass room 2.13 ms a frame against 2.18 at 7 and 2.19 at 5)
@@ -361,7 +359,7 @@ __global__ void __launch_bounds__(128, 8) k_wave_shade(DevScene s, RenderParams 
     Level *next = &w.levels[level + 1];
     if (blockIdx.x == 0 && threadIdx.x == 0) next->start = L.start + L.count;
     const uint32_t next_start = L.start + L.count;
-    const uint32_t n_iter = (L.count + blockDim.x - 1) / blockDim.x;   // whole warps iterate together
+    const uint32_t n_iter = (L.count + blockDim.x - 1) / blockDim.x;   // the block's threads iterate together
     for (uint32_t it_ = blockIdx.x; it_ < n_iter; it_ += gridDim.x) {
         const uint32_t i = it_ * blockDim.x + threadIdx.x;
         const bool active = i < L.count;
