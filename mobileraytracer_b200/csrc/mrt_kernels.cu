@@ -149,12 +149,11 @@ void launch_any(const DevScene &s, const MrtRay *rays, const float *dist, uint32
     k_trace_any<ACCEL, MODE><<<grid, 128, 0, q>>>(s, rays, dist, n, occ);
 }
 
-#define MRT_DISPATCH(fn, accel, mode, ...)                                                                 \
+// the accelerators without a persistent kernel: a thread per ray
+#define MRT_DISPATCH(fn, accel, ...)                                                                        \
     do {                                                                                                    \
         if ((accel) == MRT_ACCEL_NAIVE) fn<MRT_ACCEL_NAIVE, MRT_BVH_FAST>(__VA_ARGS__);                     \
-        else if ((accel) == MRT_ACCEL_REGULAR_GRID) fn<MRT_ACCEL_REGULAR_GRID, MRT_BVH_FAST>(__VA_ARGS__);  \
-        else if ((mode) == MRT_BVH_REFERENCE) fn<MRT_ACCEL_BVH, MRT_BVH_REFERENCE>(__VA_ARGS__);            \
-        else fn<MRT_ACCEL_BVH, MRT_BVH_FAST>(__VA_ARGS__);                                                  \
+        else fn<MRT_ACCEL_BVH, MRT_BVH_REFERENCE>(__VA_ARGS__);                                             \
     } while (0)
 
 int grid_for(const MrtContext *ctx, uint32_t n) {
@@ -187,7 +186,7 @@ int launch_trace_closest(MrtScene *s, const MrtRay *d_rays, uint32_t n, MrtHit *
         k_trace_grid_persistent<<<persistent_grid(ctx, n, kGridBlocksPerSm), 128, 0, ctx->stream>>>(s->dev, w);
         return cuda_status(ctx, cudaGetLastError(), "k_trace_grid_persistent");
     }
-    MRT_DISPATCH(launch_closest, s->opts.accelerator, s->opts.bvh_mode, s->dev, d_rays, n, d_hits, grid_for(ctx, n), ctx->stream);
+    MRT_DISPATCH(launch_closest, s->opts.accelerator, s->dev, d_rays, n, d_hits, grid_for(ctx, n), ctx->stream);
     return cuda_status(ctx, cudaGetLastError(), "k_trace_closest");
 }
 
@@ -205,7 +204,7 @@ int launch_trace_any(MrtScene *s, const MrtRay *d_rays, const float *d_dist, uin
         k_trace_any_grid<<<persistent_grid(ctx, n, kGridBlocksPerSm), 128, 0, ctx->stream>>>(s->dev, w);
         return cuda_status(ctx, cudaGetLastError(), "k_trace_any_grid");
     }
-    MRT_DISPATCH(launch_any, s->opts.accelerator, s->opts.bvh_mode, s->dev, d_rays, d_dist, n, d_occ, grid_for(ctx, n), ctx->stream);
+    MRT_DISPATCH(launch_any, s->opts.accelerator, s->dev, d_rays, d_dist, n, d_occ, grid_for(ctx, n), ctx->stream);
     return cuda_status(ctx, cudaGetLastError(), "k_trace_any");
 }
 

@@ -7,13 +7,15 @@
 // visited twice (the usual case) the kernels map threads to pixels directly, otherwise they walk an
 // explicit task list in block order, one round per repeated visit.
 //
-// NoShadows (NoShadows.cpp:19-65) has no secondary rays: one fused kernel does camera ray, closest
-// hit, shading and the running mean per pixel.
+// NoShadows (NoShadows.cpp:19-65) has no secondary rays.  On the FAST tree and the RegularGrid one launch
+// traces the camera rays and another shades a pixel's samples in order; frames with repeated visits trace all
+// their passes in one launch and fold a pixel's visits one after the other.  The other accelerators take one
+// fused kernel for camera ray, closest hit, shading and the running mean.
 //
 // Whitted and PathTracer (Whitted.cpp:17-107, PathTracer.cpp:25-164) recurse.  Here they run as a
 // wavefront over a wave of camera paths: per bounce level an extend kernel (closest hit), a shade
 // kernel that writes one node record per ray and appends shadow rays and continuation rays to
-// queues compacted with warp ballots, and an any-hit kernel for the shadow queue.  After the last
+// queues placed a block at a time, and an any-hit kernel for the shadow queue.  After the last
 // level the nodes are resolved bottom-up, level by level, combining each node's own terms with its
 // children's results in the reference's order of operations, so the per-sample value equals the
 // recursive one bit for bit.  Per-sample values are then folded into the bitmap in sample order.
@@ -736,22 +738,24 @@ void launch_noshadows(const DevScene &s, const RenderParams &p, uint32_t first, 
 template <int ACCEL, int MODE>
 void launch_wave_level(const DevScene &s, const RenderParams &p, const WaveState &w, int level, int grid, cudaStream_t q,
                        uint32_t *ctrs) {
-    if (ACCEL == MRT_ACCEL_BVH && MODE == MRT_BVH_FAST) {
+    if constexpr (ACCEL == MRT_ACCEL_BVH && MODE == MRT_BVH_FAST) {
         // counters [2 * level] and [2 * level + 1] were zeroed for this wave
         // one quorum for every level: 16 for the camera rays of level 0 made the terrain PathTracer
         // 0.4 % slower and the 256-job batch 0.4 % faster
         k_wave_extend_fast<kNodeQuorum><<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level);
-        if (w.sort_shading) k_wave_shade_sorted<<<grid, 128, 0, q>>>(s, p, w, level);
-        else k_wave_shade<<<grid, 128, 0, q>>>(s, p, w, level);
-        k_wave_shadow_fast<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level + 1);
-        return;
+    } else if constexpr (ACCEL == MRT_ACCEL_REGULAR_GRID) {
+        k_wave_extend_grid<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level);
+    } else {
+        k_wave_extend<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
     }
-    if (ACCEL == MRT_ACCEL_REGULAR_GRID) k_wave_extend_grid<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level);
-    else k_wave_extend<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
     if (w.sort_shading) k_wave_shade_sorted<<<grid, 128, 0, q>>>(s, p, w, level);
     else k_wave_shade<<<grid, 128, 0, q>>>(s, p, w, level);
-    if (ACCEL == MRT_ACCEL_REGULAR_GRID) k_wave_shadow_grid<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level + 1);
-    else k_wave_shadow<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
+    if constexpr (ACCEL == MRT_ACCEL_BVH && MODE == MRT_BVH_FAST)
+        k_wave_shadow_fast<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level + 1);
+    else if constexpr (ACCEL == MRT_ACCEL_REGULAR_GRID)
+        k_wave_shadow_grid<<<grid, 128, 0, q>>>(s, w, level, ctrs + 2 * level + 1);
+    else
+        k_wave_shadow<ACCEL, MODE><<<grid, 128, 0, q>>>(s, w, level);
 }
 
 #define MRT_DISPATCH(fn, accel, mode, ...)                                                                 \
