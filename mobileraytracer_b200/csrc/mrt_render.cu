@@ -642,45 +642,59 @@ bool plan_tasks(const MrtRenderOpts &o, uint32_t stride_px, TaskPlan &plan) {
     if (bsx == 0 || bsy == 0) return false;
     const uint32_t domain = (w / bsx) * (h / bsy);
     const uint64_t res = (uint64_t)w * h;
-    // Every visit of a pixel goes to the round of its number (a round renders a pixel at most once), block
-    // order kept per pixel; tasks outside the bitmap (undefined behaviour in the reference) are dropped.
-    const size_t n_px = (size_t)stride_px * h;
-    constexpr uint32_t kNone = 0xFFFFFFFFu;
-    std::vector<std::vector<uint2>> rounds;      // by round and bitmap pixel (x = kNone: not rendered)
-    std::vector<uint32_t> round_size, visits(n_px, 0);
-    uint64_t n_all = 0;
-    bool inside = true;   // every task in the rectangle [0, w) x [0, rows)
+    // the block rows: bsx pixels from (sx, y), in block order
     const uint32_t rows = 16u * bsy;
+    std::vector<uint2> spans;
+    spans.reserve(256u * (size_t)bsy);
+    bool inside = true;   // every task in the rectangle [0, w) x [0, rows)
     for (uint32_t i = 0; i < 256; ++i) {
         const float block = halton(i, 2);
         const uint32_t rb = (uint32_t)roundf(block * (float)domain);
         const uint32_t pixel = (uint32_t)(((uint64_t)rb * bsx) % res);
         const uint32_t sy = ((pixel / w) * bsy) % h;
         for (uint32_t y = sy; y < sy + bsy; ++y) {
-            const uint32_t yw = y * stride_px;
-            const uint32_t sx = (pixel + yw) % w;
-            n_all += bsx;
+            const uint32_t sx = (pixel + y * stride_px) % w;
             inside = inside && y < rows && sx + bsx <= w;
-            for (uint32_t x = sx; x < sx + bsx; ++x) {
-                const uint32_t index = yw + x;
-                if ((uint64_t)index >= (uint64_t)n_px) continue;
-                const uint32_t r = visits[index]++;
-                if (r >= rounds.size()) {
-                    rounds.emplace_back(n_px, make_uint2(kNone, 0u));
-                    round_size.push_back(0);
-                }
-                rounds[r][index] = make_uint2(x, y);
-                ++round_size[r];
-            }
+            spans.push_back(make_uint2(sx, y));
         }
     }
-    // the implicit rectangle?
-    if (inside && n_all == (uint64_t)w * rows && rounds.size() == 1 && round_size[0] == n_all) {
-        plan.implicit = true;
-        plan.n_tasks = w * rows;
-        plan.round_first = {0};
-        plan.round_count = {plan.n_tasks};
-        return true;
+    // The implicit rectangle?  As many pixels as it has, all in it and none twice: looked up by block row, the
+    // pixels themselves are not walked (first 1920x1080 frame of a scene: 19.5 ms with a walk, 9.4 with a walk of a
+    // list of the pixels, 1.8 so).
+    if (inside && spans.size() * (size_t)bsx == (size_t)w * rows) {
+        std::vector<uint64_t> by_row;   // y << 32 | x
+        by_row.reserve(spans.size());
+        for (const uint2 &span : spans) by_row.push_back((uint64_t)span.y << 32 | span.x);
+        std::sort(by_row.begin(), by_row.end());
+        bool once = true;
+        for (size_t k = 1; k < by_row.size() && once; ++k) once = by_row[k] >= by_row[k - 1] + bsx;
+        if (once) {
+            plan.implicit = true;
+            plan.n_tasks = w * rows;
+            plan.round_first = {0};
+            plan.round_count = {plan.n_tasks};
+            return true;
+        }
+    }
+    // Every visit of a pixel goes to the round of its number (a round renders a pixel at most once), block
+    // order kept per pixel; tasks outside the bitmap (undefined behaviour in the reference) are dropped.
+    const size_t n_px = (size_t)stride_px * h;
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    std::vector<std::vector<uint2>> rounds;      // by round and bitmap pixel (x = kNone: not rendered)
+    std::vector<uint32_t> round_size, visits(n_px, 0);
+    for (const uint2 &span : spans) {
+        const uint32_t yw = span.y * stride_px;
+        for (uint32_t x = span.x; x < span.x + bsx; ++x) {
+            const uint32_t index = yw + x;
+            if ((uint64_t)index >= (uint64_t)n_px) continue;
+            const uint32_t r = visits[index]++;
+            if (r >= rounds.size()) {
+                rounds.emplace_back(n_px, make_uint2(kNone, 0u));
+                round_size.push_back(0);
+            }
+            rounds[r][index] = make_uint2(x, span.y);
+            ++round_size[r];
+        }
     }
     plan.implicit = false;
     // a round's order is free: 2x16-pixel tiles of the bitmap, one after the other, so that the 32 rays a
