@@ -26,6 +26,13 @@ namespace mrt {
 // Whitted frame 105.6 us; 4: 104.3, 8: 64 registers and 506 bytes of spills, 115; batches of 11 and 12 soups
 // 0.633 and 2.59 ms at 5, 0.643 and 2.66 at 4, 0.667 and 2.63 at 8)
 constexpr int kPathBlocksPerSm = 5;
+// and for PathTracer frames of a few triangles with a path for every lane, whose tree leaves L1 to the lanes'
+// frames so that more warps hide more of their latency: the glass room at 512x512 (3 triangles) takes 1.91 ms
+// at 5 blocks, 1.78 at 6, 1.69 at 7, 1.71 at 8, the Cornell box at 640x288 with four light samples 1.80, 1.67,
+// 1.64 and 1.68.  Not beyond: terrains of 200 and 600 triangles 0.76 and 1.09 ms at 5, 0.78 and 1.10 at 7, Whitted
+// frames of both rooms 2 to 3 % slower at 7, 129,536 paths (fewer than the lanes) the same.
+constexpr int kSmallPathBlocksPerSm = 7;
+constexpr uint32_t kSmallPathTriangles = 64;
 constexpr int kPathFrames = 12;   // recursion depth a lane can hold: depth_max + 1 <= kPathFrames
 
 struct PathFrame {

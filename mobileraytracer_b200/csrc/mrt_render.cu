@@ -567,7 +567,8 @@ struct WavePathWork {
     }
 };
 
-__global__ void __launch_bounds__(128, kPathBlocksPerSm) k_wave_paths(DevScene s, RenderParams p, WaveState w, uint32_t *ctr) {
+template <int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) k_wave_paths(DevScene s, RenderParams p, WaveState w, uint32_t *ctr) {
     WavePathWork work{&s, &p, w, ctr};
     persistent_paths(work);
 }
@@ -1102,7 +1103,12 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
                 if (paths) {
                     if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
-                    k_wave_paths<<<ctx->sm_count * kPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
+                    const bool small = o->shader == MRT_SHADER_PATHTRACER && s->n_tri <= kSmallPathTriangles &&
+                                       w.n_roots >= (uint32_t)ctx->sm_count * kSmallPathBlocksPerSm * 128u;
+                    if (small)
+                        k_wave_paths<kSmallPathBlocksPerSm><<<ctx->sm_count * kSmallPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
+                    else
+                        k_wave_paths<kPathBlocksPerSm><<<ctx->sm_count * kPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);
                     launches += 2;   // with the fold below
                 } else {
                     cudaMemsetAsync(w.levels, 0, sizeof(Level) * (levels + 2), wq);

@@ -1,6 +1,7 @@
 """Queues of the wavefront's shade kernel (places per block, continuation rays ordered by octant): levels of
 a few rays up to many blocks, several children and light samples per ray, against mrt_render's
-whole-path launch, which has no queues: the same words (GPU)."""
+whole-path launch, which has no queues (the last sizes on both sides of the path count from which PathTracer
+frames of few triangles take more blocks): the same words (GPU)."""
 import ctypes
 
 import pytest
@@ -11,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shader", [capi.MRT_SHADER_WHITTED, capi.MRT_SHADER_PATHTRACER])
-@pytest.mark.parametrize("w,h,spp,spl", [(16, 16, 1, 1), (16, 16, 7, 4), (48, 32, 1, 3), (112, 48, 2, 2)])
+@pytest.mark.parametrize("w,h,spp,spl", [(16, 16, 1, 1), (16, 16, 7, 4), (48, 32, 1, 3), (112, 48, 2, 2), (352, 368, 1, 1), (368, 368, 1, 2)])
 def test_queued_levels_equal_whole_paths(ctx, shader, w, h, spp, spl):
     torch = pytest.importorskip("torch")
     sc = scenes.glass_room()
