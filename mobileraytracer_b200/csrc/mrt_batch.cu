@@ -214,7 +214,9 @@ struct BatchPathWork {
     }
 };
 
-__global__ void __launch_bounds__(128, kPathBlocksPerSm) k_batch_paths(BatchState b) {
+constexpr uint32_t kSmallBatchBlocksPerSm = 8;   // path_blocks()
+template <int kBlocks>
+__global__ void __launch_bounds__(128, kBlocks) k_batch_paths(BatchState b) {
     BatchPathWork work{b, b.work};
     persistent_paths(work);
 }
@@ -463,7 +465,7 @@ void launch_traversal(const BatchState &s, int level, int grid, cudaStream_t q, 
 }
 
 // the wave up to the per-sample values: camera rays, every bounce level, the bottom-up resolve
-// (threads = 0: whole paths in one persistent launch instead)
+// (threads = 0: whole paths in one persistent launch instead, of bps = path_blocks() blocks per SM)
 void launch_trace_kernels(MrtBatch *b, int pipe, uint32_t threads, uint32_t bps, cudaStream_t q) {
     const BatchState s = state_of(b, pipe);
     const int sm = b->ctx->sm_count;
@@ -471,7 +473,8 @@ void launch_trace_kernels(MrtBatch *b, int pipe, uint32_t threads, uint32_t bps,
     const int grid = sm * 16;
     if (threads == 0) {
         k_batch_begin<<<1, 64, 0, q>>>(s);
-        k_batch_paths<<<sm * kPathBlocksPerSm, 128, 0, q>>>(s);
+        if (bps == kSmallBatchBlocksPerSm) k_batch_paths<kSmallBatchBlocksPerSm><<<sm * kSmallBatchBlocksPerSm, 128, 0, q>>>(s);
+        else k_batch_paths<kPathBlocksPerSm><<<sm * kPathBlocksPerSm, 128, 0, q>>>(s);
         return;
     }
     auto trav = [&](int level, bool extend) {
@@ -579,6 +582,16 @@ bool whole_paths_wave(const WaveDesc &d) {
     return 2ull * largest < d.n_roots;
 }
 
+// blocks per SM of a whole-path wave: the rule of mrt_render's frames, for all of the wave's jobs, with 8 blocks
+// where a frame takes 7 (PathTracer batches of 16 Cornell boxes and of 16 glass rooms at 256x256, two light
+// samples: 8.02 and 11.6 ms at 5 blocks, 7.70 and 11.2 at 6, 8.02 and 11.0 at 7, 7.63 and 10.6 at 8)
+uint32_t path_blocks(const MrtBatch *b, const WaveDesc &d) {
+    bool small = d.n_roots >= (uint32_t)b->ctx->sm_count * kSmallBatchBlocksPerSm * 128u;
+    for (uint32_t k = 0; small && k < d.n_seg; ++k)
+        small = small_paths(b->h_jobs[d.seg[k].job].shader, b->h_scenes[d.seg[k].job].n_tri);
+    return small ? kSmallBatchBlocksPerSm : kPathBlocksPerSm;
+}
+
 // one wave on pipeline `pipe`: description copy, the traced part (a graph replay), then the fold
 // into the bitmaps, which waits for the previous wave's fold (a pixel's samples may straddle the
 // two waves, and their order must stay the sample order)
@@ -586,6 +599,7 @@ int run_wave(MrtBatch *b, const WaveDesc &d, int pipe, uint32_t threads, uint32_
     MrtContext *ctx = b->ctx;
     BatchPipe &P = b->pipes[pipe];
     cudaStream_t q = P.stream;
+    if (threads == 0) bps = path_blocks(b, d);
     if (P.jobs_seen != b->jobs_uploaded) {
         cudaStreamWaitEvent(q, b->ev_jobs, 0);
         P.jobs_seen = b->jobs_uploaded;
@@ -980,7 +994,6 @@ int mrt_batch_step(MrtBatch *b, uint32_t max_waves, uint32_t *launched) {
         uint32_t threads = b->block_threads, bps = b->blocks_per_sm;
         if (b->opts.kernel == 0 && b->n_levels <= kPathFrames && whole_paths_wave(d)) {
             threads = 0;
-            bps = 8;
             ++b->waves_paths;
         }
         st = run_wave(b, d, pipe, threads, bps, r, w > b->waves_done ? (int)((w - 1) % kRing) : -1);

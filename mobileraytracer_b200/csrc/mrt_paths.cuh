@@ -33,6 +33,7 @@ constexpr int kPathBlocksPerSm = 5;
 // frames of both rooms 2 to 3 % slower at 7, 129,536 paths (fewer than the lanes) the same.
 constexpr int kSmallPathBlocksPerSm = 7;
 constexpr uint32_t kSmallPathTriangles = 64;
+inline bool small_paths(int32_t shader, uint32_t n_tri) { return shader == MRT_SHADER_PATHTRACER && n_tri <= kSmallPathTriangles; }
 constexpr int kPathFrames = 12;   // recursion depth a lane can hold: depth_max + 1 <= kPathFrames
 
 struct PathFrame {

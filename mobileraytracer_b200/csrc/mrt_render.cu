@@ -1103,7 +1103,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
                 if (paths) {
                     if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
-                    const bool small = o->shader == MRT_SHADER_PATHTRACER && s->n_tri <= kSmallPathTriangles &&
+                    const bool small = small_paths(o->shader, s->n_tri) &&
                                        w.n_roots >= (uint32_t)ctx->sm_count * kSmallPathBlocksPerSm * 128u;
                     if (small)
                         k_wave_paths<kSmallPathBlocksPerSm><<<ctx->sm_count * kSmallPathBlocksPerSm, 128, 0, q>>>(s->dev, p, w, ctx->d_counters);

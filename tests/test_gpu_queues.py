@@ -6,7 +6,7 @@ import ctypes
 
 import pytest
 
-from mobileraytracer_b200 import Scene, capi, scenes
+from mobileraytracer_b200 import Batch, Scene, capi, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +32,22 @@ def test_queued_levels_equal_whole_paths(ctx, shader, w, h, spp, spl):
         out.append((bm, acc, st.rays_closest, st.rays_shadow))
     assert out[0][2:] == out[1][2:]
     assert torch.equal(out[0][0], out[1][0]) and torch.equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("jobs,soup", [(2, False), (3, False), (3, True)])
+def test_batches_of_small_scenes_equal_frames(ctx, jobs, soup):
+    """Waves below and above the path count of the small-scene launch, and one with a larger scene among them."""
+    torch = pytest.importorskip("torch")
+    batch, want = Batch(ctx, max_depth=6, max_spl=2), []
+    for i in range(jobs):
+        sc = scenes.triangle_soup(500, 3, 256, 256) if soup and i == 1 else scenes.glass_room()
+        g = Scene(ctx, sc).build(capi.MRT_ACCEL_BVH)
+        opts = capi.render_opts(shader=capi.MRT_SHADER_PATHTRACER, width=256, height=256, spp=1, spl=2, seed=i, depth_min=2, depth_max=6)
+        got, frame = (torch.zeros(256, 256, dtype=torch.int32, device="cuda") for _ in range(2))
+        g.render(sc.camera, opts, bitmap=frame)
+        batch.submit(g, sc.camera, opts, got)
+        want.append((g, got, frame))
+    batch.run()
+    batch.completed()
+    torch.cuda.synchronize()
+    assert all(torch.equal(got, frame) for _, got, frame in want)
