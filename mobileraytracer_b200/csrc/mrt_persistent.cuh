@@ -1,7 +1,7 @@
 // mrt_persistent.cuh - persistent closest-hit engine for the FAST BVH.
 //
 // Rays in a warp need very different amounts of work (a camera ray that misses the scene ends at
-// the root box, one that crosses a dense soup visits ~60 node pairs), so a one-ray-per-thread
+// the root box, one that crosses a dense soup visits ~28 wide nodes), so a one-ray-per-thread
 // kernel leaves most lanes idle behind the warp's longest ray.  Here every lane carries a
 // resumable traversal state and the warp loops:
 //   1. refill: lanes whose work item is finished take new items from a global counter, one
@@ -23,9 +23,9 @@ namespace mrt {
 // the node phase of a warp ends when no lane searches any more, or when fewer than Q lanes search
 // while others hold leaves: those leaves are tested first, and the few searching lanes go on in the
 // next node phase.  Coherent camera rays do best with Q = 16 (the NoShadows trace of the
-// 1,000,000-triangle soup frame: 1757 Mrays/s against 1757 at 20, 1715 at 24, 1575 at 32, 1610 at
-// 8), the incoherent bounces of the wavefront with Q = 4 (terrain PathTracer: 3, 4 and 6 within
-// 0.3 %, 8 1.5 % slower).
+// 1,000,000-triangle soup frame before the packed node test: 1757 Mrays/s against 1757 at 20, 1715 at
+// 24, 1575 at 32, 1610 at 8; with it 12 and 20 are no better than 16 either), the incoherent bounces
+// of the wavefront with Q = 4 (terrain PathTracer: 3, 4 and 6 within 0.3 %, 8 1.5 % slower).
 #ifndef MRT_NODE_QUORUM
 #define MRT_NODE_QUORUM 4
 #endif

@@ -228,7 +228,9 @@ __global__ void __launch_bounds__(128, kGridBlocksPerSm) k_ns_trace_grid(DevScen
 // shading of items j0 .. j0 + n_pix - 1 of a traced chunk: the hit of sample si of item j0 + j is
 // hits[si * hit_stride + j] (hit_stride = the chunk's item count; a band of the chunk passes the hits
 // from its first item on)
-__global__ void __launch_bounds__(128) k_ns_shade(DevScene s, RenderParams p, uint32_t first, uint32_t j0, uint32_t n_pix,
+// (10 blocks per SM: the kernel waits for scattered triangle records, so more warps pay; a 1080p soup frame
+// 1,130 us without a bound, 7 blocks and 71 registers, 1,123 at 8, 1,120 at 10, 1,120 at 12)
+__global__ void __launch_bounds__(128, 10) k_ns_shade(DevScene s, RenderParams p, uint32_t first, uint32_t j0, uint32_t n_pix,
                                                   uint32_t s0, uint32_t n_s, uint32_t tiles_x, const uint2 *__restrict__ hits,
                                                   uint32_t hit_stride) {
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < n_pix; j += gridDim.x * blockDim.x) {
