@@ -31,7 +31,7 @@ def orc() -> ctypes.CDLL:
     if _orc is None:
         path = os.path.join(REF_DIR, "liborc.so")
         if not os.path.exists(path):
-            raise RuntimeError(f"{path} missing: run `make -C oracle orc`")
+            raise ReferenceMissing(f"{path} missing: run `make -C oracle orc`")
         lib = ctypes.CDLL(path)
         vp, fp, ip = ctypes.c_void_p, ctypes.POINTER(ctypes.c_float), ctypes.c_int
         _declare(lib, {
@@ -68,12 +68,16 @@ def orc() -> ctypes.CDLL:
     return _orc
 
 
+class ReferenceMissing(RuntimeError):
+    """The library of the reference's own compiled sources was not built (no reference checkout here)."""
+
+
 def ref(fast: bool = False) -> ctypes.CDLL:
     key = "fast" if fast else "parity"
     if key not in _ref:
         path = os.path.join(REF_DIR, "liboracle_ref_fast.so" if fast else "liboracle_ref.so")
         if not os.path.exists(path):
-            raise RuntimeError(f"{path} missing: run `make -C oracle ref` where the reference checkout exists")
+            raise ReferenceMissing(f"{path} missing: run `make -C oracle ref` where the reference checkout exists")
         lib = ctypes.CDLL(path)
         vp, fp, ip = ctypes.c_void_p, ctypes.POINTER(ctypes.c_float), ctypes.c_int
         dp = ctypes.POINTER(ctypes.c_double)

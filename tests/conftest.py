@@ -14,6 +14,16 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: several seconds of CPU work in the oracle")
 
 
+@pytest.hookimpl(wrapper=True)
+def pytest_pyfunc_call(pyfuncitem):
+    """Tests against the reference's own compiled sources skip, with the reason, where these are not built."""
+    import orc
+    try:
+        return (yield)
+    except orc.ReferenceMissing as e:
+        pytest.skip(str(e))
+
+
 @pytest.fixture(scope="session")
 def ctx():
     import mobileraytracer_b200 as m
