@@ -714,6 +714,7 @@ int build_fast_bvh(MrtScene *s) {
         st = cuda_status(ctx, cudaGetLastError(), "fast bvh kernels");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "fast bvh build");
     }
+    if (st != MRT_OK) drain(ctx);
     DevBuf *tmp[] = {&cb, &keys[0], &keys[1], &vals[1 - cur], &hist, &total, &pint, &pleaf, &ctr};
     for (DevBuf *b : tmp) dev_free(*b);
     // collapse into 8-wide compressed nodes, level by level, from the root
@@ -763,6 +764,7 @@ int build_fast_bvh(MrtScene *s) {
                                                   cudaMemcpyDeviceToDevice, q), "collapse copy");
         if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "collapse copy");
     }
+    if (st != MRT_OK) drain(ctx);
     DevBuf *tmp2[] = {&wide, &queue[0], &queue[1], &wctr, &bmin, &bmax, &vals[cur], &lft, &rgt, &fst, &lst, &imin, &imax, &costs};
     for (DevBuf *b : tmp2) dev_free(*b);
     if (st != MRT_OK) return st;

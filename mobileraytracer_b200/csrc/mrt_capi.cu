@@ -82,8 +82,9 @@ static void arena_free(MrtArena *a, void *p, size_t bytes) {
 // cudaFree, each of which maps memory and waits for the device, a 200,003-triangle scene took 16 to 57 ms
 // to upload, build and render once, of which the kernels are 0.9 ms.  The pool keeps at most kPoolKeep
 // unused bytes (trim_pool, after builds and when scenes go) and none once the device's last context is
-// gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight (for a pooled
-// buffer cudaFree does not wait).  Larger buffers are few and long-lived (ray pools) and would only make the
+// gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight.  For a pooled
+// buffer cudaFree does not wait, and another context may be given the memory at once, so whoever frees waits
+// first: calls that end in an error with work queued, and a buffer replaced by a larger one (drain).  Larger buffers are few and long-lived (ray pools) and would only make the
 // pool's bound meaningless.
 constexpr size_t kPoolMost = 256u << 20, kPoolKeep = 1u << 30;
 struct DevicePool {
@@ -126,7 +127,13 @@ void trim_pool(MrtContext *ctx) {
     if (reserved - used > kPoolKeep) cudaMemPoolTrimTo(ctx->pool, (size_t)used + kPoolKeep);
 }
 
+void drain(MrtContext *ctx) {
+    for (cudaStream_t q : {ctx->stream, ctx->copy_stream, ctx->wave_stream})
+        if (q) cudaStreamSynchronize(q);
+}
+
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
+    if (b.ptr) drain(ctx);
     dev_free(b);
     if (bytes == 0) bytes = 16;
     if (ctx->arena) {
@@ -325,9 +332,7 @@ int mrt_context_create(int device, MrtContext **out) {
 void mrt_context_destroy(MrtContext *ctx) {
     if (!ctx) return;
     cudaSetDevice(ctx->device);
-    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
-    if (ctx->copy_stream) cudaStreamSynchronize(ctx->copy_stream);
-    if (ctx->wave_stream) cudaStreamSynchronize(ctx->wave_stream);
+    drain(ctx);
     for (auto &b : ctx->scratch) dev_free(b);
     for (auto &b : ctx->wave) dev_free(b);
     for (auto &b : ctx->raster) dev_free(b);
@@ -427,6 +432,11 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
         set_error(ctx, "mrt_scene_create: more than 2^30 primitives of one type");
         return MRT_ERR_ARG;
     }
+    for (uint32_t k = 0; k < d->n_lights; ++k)
+        if (d->lights[k].kind != MRT_LIGHT_POINT && d->lights[k].kind != MRT_LIGHT_AREA) {
+            set_error(ctx, "mrt_scene_create: invalid light kind");
+            return MRT_ERR_ARG;
+        }
     cudaSetDevice(ctx->device);
     MrtScene *s = new (std::nothrow) MrtScene();
     if (!s) return MRT_ERR_OOM;
@@ -511,7 +521,6 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
         const MrtMaterial &m = l.radiance;
         o.radiance = DevMaterial{V3{m.le[0], m.le[1], m.le[2]}, V3{m.kd[0], m.kd[1], m.kd[2]},
                                  V3{m.ks[0], m.ks[1], m.ks[2]}, V3{m.kt[0], m.kt[1], m.kt[2]}, m.ior};
-        if (l.kind != MRT_LIGHT_POINT && l.kind != MRT_LIGHT_AREA) st = MRT_ERR_ARG;
     }
     std::vector<DevMaterial> hm(s->n_mat);
     for (uint32_t i = 0; i < s->n_mat; ++i) {
@@ -530,9 +539,9 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
     up(s->lights, hl.data(), sizeof(DevLight) * s->n_light);
     up(s->mats, hm.data(), sizeof(DevMaterial) * s->n_mat);
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "scene upload");
+    if (st != MRT_OK) drain(ctx);
     dev_free(st_abc); dev_free(st_n); dev_free(st_c); dev_free(st_m);
     if (st != MRT_OK) {
-        if (ctx->error.empty()) set_error(ctx, "mrt_scene_create: invalid light kind");
         scene_free(s);
         delete s;
         return st;
@@ -598,7 +607,7 @@ int mrt_scene_build(MrtScene *s, const MrtAccelOpts *o) {
         if (o->camera) camera_box(*o->camera, cmn, cmx);
         st = build_grids(s, cmn, cmx, o->grid_size, o->grid_index);
     }
-    if (st != MRT_OK) return st;
+    if (st != MRT_OK) { drain(ctx); return st; }
     st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_scene_build");
     trim_pool(ctx);
     if (st == MRT_OK) s->built = true;

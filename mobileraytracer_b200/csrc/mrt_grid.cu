@@ -420,6 +420,7 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
                 s->grid_refs_count[type] = total;
             }
         }
+        if (st != MRT_OK) drain(ctx);
         dev_free(count); dev_free(fill); dev_free(sums); dev_free(offs);
         // the cell records and the skip bits, along the strides the walks read with
         g.id_mask = 0xFFFFFFFFu;
@@ -442,6 +443,7 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
             st = cuda_status(ctx, cudaGetLastError(), "grid cells");
             if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "grid cells");
         }
+        if (st != MRT_OK) drain(ctx);
         dev_free(start_buf); dev_free(reach);
         if (st != MRT_OK) return st;
         g.cells = (const uint2 *)s->grid_cells[type].ptr;

@@ -116,6 +116,7 @@ int cuda_status(MrtContext *ctx, cudaError_t e, const char *what);
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int ensure(MrtContext *ctx, DevBuf &b, size_t bytes);   // grow-only scratch
+void drain(MrtContext *ctx);                            // waits for all work of the context's streams
 int check_kernel_error(MrtContext *ctx);                // waits for the stream, reads and clears the error flag
 void trim_pool(MrtContext *ctx);                        // gives memory beyond the pool's bound back
 
