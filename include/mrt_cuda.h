@@ -243,19 +243,21 @@ void *mrt_context_stream(MrtContext *ctx);
  * (geometry, trees, build scratch) and their render scratch: scenes come and go without cudaMalloc /
  * cudaFree, so building or evicting a scene never synchronises the device while other work runs, and
  * the sum of all resident scenes is bounded by the arena's size.  Several contexts on one device may
- * share an arena (e.g. one building scenes while another renders); it is thread-safe.  Freeing a
- * scene returns its blocks at once: destroy a scene only when no work that reads it is in flight. */
+ * share an arena (e.g. one building scenes while another renders); it is thread-safe. */
 int mrt_arena_create(int device, uint64_t bytes, MrtArena **out);
 /* MRT_ERR_STATE (and nothing freed) while buffers carved from the arena are alive. */
 int mrt_arena_destroy(MrtArena *arena);
 int mrt_arena_stats(MrtArena *arena, uint64_t *capacity, uint64_t *used, uint64_t *peak,
                     uint64_t *largest_free);
-/* Later device allocations of ctx come from `arena` (NULL: cudaMalloc again); existing buffers keep
- * their origin. */
+/* Later device allocations of ctx come from `arena` (NULL: from the device's memory pool or cudaMalloc
+ * again); existing buffers keep their origin. */
 int mrt_context_set_arena(MrtContext *ctx, MrtArena *arena);
 
 /* ---- scene ---------------------------------------------------------------------------------- */
 int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *desc, MrtScene **out);
+/* Destroying a scene, or building it again, returns its buffers at once, for any context to use.  Both wait
+ * for the scene's context and, while a batch has unfinished jobs on the scene, for the device; waves that
+ * start later would read freed memory, so a scene stays as it is until its jobs are reported done. */
 void mrt_scene_destroy(MrtScene *scene);
 int mrt_scene_build(MrtScene *scene, const MrtAccelOpts *opts);
 /* Hand a scene to another context on the same device (e.g. from a context that builds scenes on one

@@ -416,6 +416,7 @@ struct MrtBatch {
         uint64_t total = 0;          // paths
         uint64_t next = 0;           // next path to schedule
         bool live = false;
+        std::shared_ptr<int> scene;  // MrtScene::in_use while live
     };
     std::vector<Job> slots;          // [max_jobs], slot = id % max_jobs
     std::vector<uint32_t> active;    // slots with paths left, submission order
@@ -640,6 +641,7 @@ int retire(MrtBatch *b, bool wait_one) {
         if (it != b->finishing.end()) {
             for (uint32_t slot : it->second) {
                 b->slots[slot].live = false;
+                b->slots[slot].scene.reset();
                 b->newly_done.push_back(b->slots[slot].id);
                 ++b->jobs_done;
             }
@@ -771,16 +773,17 @@ int autotune(MrtBatch *b) {
 
 void free_batch(MrtBatch *b) {
     if (!b) return;
+    for (BatchPipe &P : b->pipes)
+        if (P.stream) cudaStreamSynchronize(P.stream);
+    drain(b->ctx);
     for (uint32_t p = 0; p < kMaxPipes; ++p) {
         BatchPipe &P = b->pipes[p];
-        if (P.stream) cudaStreamSynchronize(P.stream);
         for (auto &kv : P.graphs) cudaGraphExecDestroy(kv.second);
         DevBuf *bufs[] = {&P.d_desc, &P.d_rays, &P.d_nodes, &P.d_shadows, &P.d_levels, &P.d_root_rgb, &P.d_root_job,
                           &P.d_root_local, &P.d_work};
         for (DevBuf *x : bufs) dev_free(*x);
         if (P.stream) cudaStreamDestroy(P.stream);
     }
-    if (b->ctx && b->ctx->stream) cudaStreamSynchronize(b->ctx->stream);
     dev_free(b->d_jobs);
     dev_free(b->d_scenes);
     dev_free(b->d_counters);
@@ -961,6 +964,7 @@ int mrt_batch_submit(MrtBatch *b, const MrtBatchJob *job, uint64_t *job_id) {
     j.total = total;
     j.next = 0;
     j.live = true;
+    j.scene = s->in_use;
     b->active.push_back(slot);
     if (job_id) *job_id = j.id;
     return MRT_OK;

@@ -84,7 +84,8 @@ static void arena_free(MrtArena *a, void *p, size_t bytes) {
 // unused bytes (trim_pool, after builds and when scenes go) and none once the device's last context is
 // gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight.  For a pooled
 // buffer cudaFree does not wait, and another context may be given the memory at once, so whoever frees waits
-// first: calls that end in an error with work queued, and a buffer replaced by a larger one (drain).  Larger buffers are few and long-lived (ray pools) and would only make the
+// first (drain): calls that end in an error with work queued, a buffer replaced by a larger one, a scene destroyed
+// or built again.  Larger buffers are few and long-lived (ray pools) and would only make the
 // pool's bound meaningless.
 constexpr size_t kPoolMost = 256u << 20, kPoolKeep = 1u << 30;
 struct DevicePool {
@@ -130,6 +131,11 @@ void trim_pool(MrtContext *ctx) {
 void drain(MrtContext *ctx) {
     for (cudaStream_t q : {ctx->stream, ctx->copy_stream, ctx->wave_stream})
         if (q) cudaStreamSynchronize(q);
+}
+
+void drain(MrtScene *s) {
+    if (s->in_use.use_count() > 1) cudaDeviceSynchronize();   // (as every cudaFree of a plain allocation)
+    else cudaStreamSynchronize(s->ctx->stream);
 }
 
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
@@ -561,7 +567,7 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
 void mrt_scene_destroy(MrtScene *s) {
     if (!s) return;
     cudaSetDevice(s->ctx->device);
-    cudaStreamSynchronize(s->ctx->stream);
+    drain(s);
     scene_free(s);
     trim_pool(s->ctx);
     delete s;
@@ -592,6 +598,7 @@ int mrt_scene_build(MrtScene *s, const MrtAccelOpts *o) {
     }
     s->built = false;
     s->opts = *o;
+    drain(s);
     dev_free(s->fnodes);
     dev_free(s->ftris);
     for (int k = 0; k < 3; ++k) { dev_free(s->rnodes[k]); dev_free(s->grid_cells[k]); dev_free(s->grid_refs[k]); }

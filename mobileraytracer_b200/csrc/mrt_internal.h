@@ -5,6 +5,7 @@
 
 #include <atomic>
 #include <map>
+#include <memory>
 #include <mutex>
 #include <cstdint>
 #include <cstdio>
@@ -98,6 +99,8 @@ struct MrtScene {
     std::vector<float> h_tri;           // A, AB, AC per triangle (host_triangles; empty until a build asks for it)
     std::vector<float> h_sph;           // 4 per sphere
     std::vector<float> h_pln;           // 6 per plane (point, normalised normal)
+    // held by every unfinished job of a batch (mrt_batch.cu): its waves read the scene on their own streams
+    std::shared_ptr<int> in_use = std::make_shared<int>(0);
     // render state
     std::atomic<uint32_t> progress{0};
     std::atomic<int> stop{0};
@@ -117,6 +120,7 @@ int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
 int ensure(MrtContext *ctx, DevBuf &b, size_t bytes);   // grow-only scratch
 void drain(MrtContext *ctx);                            // waits for all work of the context's streams
+void drain(MrtScene *s);                                // and for batches with jobs on the scene
 int check_kernel_error(MrtContext *ctx);                // waits for the stream, reads and clears the error flag
 void trim_pool(MrtContext *ctx);                        // gives memory beyond the pool's bound back
 

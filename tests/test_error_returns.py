@@ -1,4 +1,4 @@
-"""Calls that fail half-way, on the library's own host code over a stand-in for the CUDA runtime (tests/cpp/
+"""Calls that fail half-way and scenes that go while a batch reads them, on the library's own host code over a stand-in for the CUDA runtime (tests/cpp/
 fake_cuda.cpp; no GPU): buffers of the device's pool are only freed once nothing queued uses them."""
 import os
 import subprocess
@@ -8,7 +8,7 @@ import pytest
 from mobileraytracer_b200 import build as B
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SOURCES = ["mrt_capi.cu", "mrt_bvh.cu", "mrt_grid.cu", "mrt_kernels.cu"]
+SOURCES = ["mrt_capi.cu", "mrt_bvh.cu", "mrt_grid.cu", "mrt_kernels.cu", "mrt_batch.cu"]
 
 
 @pytest.fixture(scope="module")
@@ -39,3 +39,7 @@ def _run(objects, name):
 
 def test_scene_creation_and_builds_that_fail(objects):
     _run(objects, "error_returns")
+
+
+def test_scenes_that_go_while_a_batch_reads_them(objects):
+    _run(objects, "scene_in_use")
