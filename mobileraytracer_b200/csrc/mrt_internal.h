@@ -69,7 +69,8 @@ struct MrtContext {
     DevBuf scratch[4];
     MrtArena *arena = nullptr;          // device allocations of this context come from here when set
     // render scratch shared by the context's scenes (renders on one context are serialised on its
-    // stream): wavefront queues, per-sample values, host-path bitmap staging
+    // stream): wavefront queues, per-sample values, the pixels a paired wavefront started from, host-path
+    // bitmap staging
     DevBuf wave[8];
     // raster preview scratch: depth keys, queued large triangles, counters, host-path bitmap, overflow lists
     DevBuf raster[5];

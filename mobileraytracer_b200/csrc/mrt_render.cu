@@ -610,7 +610,7 @@ __global__ void k_wave_accumulate(RenderParams p, WaveState w) {
     const uint32_t g0 = w.root_first, g1 = w.root_first + w.n_roots;
     const uint32_t t0 = g0 / p.spp, t1 = (g1 - 1) / p.spp;
     for (uint32_t t = t0 + blockIdx.x * blockDim.x + threadIdx.x; t <= t1; t += gridDim.x * blockDim.x) {
-        const Task k = task_of(p, p.task_base + t);
+        const Task k = task_of(p, p.task_base + wave_task(w, t));
         const int64_t slot = p.accum ? accum_slot(p, k) : -1;
         uint32_t bm = p.bitmap[k.index];
         float4 acc = slot >= 0 ? p.accum[slot] : make_float4(0, 0, 0, 0);
@@ -633,6 +633,7 @@ struct TaskPlan {
     bool uploaded = false;               // explicit list already in the scene's work[0]
     bool implicit = true;
     uint32_t n_tasks = 0;
+    size_t end = 0;                      // bitmap pixels up to the last task's
     std::vector<uint2> list;                 // explicit tasks (x, y) by round
     std::vector<uint32_t> next_visit;        // the same pixel's task in the next round (kNoTask: none)
     std::vector<uint32_t> round_first, round_count;
@@ -674,6 +675,7 @@ bool plan_tasks(const MrtRenderOpts &o, uint32_t stride_px, TaskPlan &plan) {
         if (once) {
             plan.implicit = true;
             plan.n_tasks = w * rows;
+            plan.end = (size_t)(rows - 1) * stride_px + w;
             plan.round_first = {0};
             plan.round_count = {plan.n_tasks};
             return true;
@@ -695,6 +697,7 @@ bool plan_tasks(const MrtRenderOpts &o, uint32_t stride_px, TaskPlan &plan) {
                 plan.round_count.push_back(0);
             }
             ++plan.round_count[r];
+            plan.end = std::max(plan.end, at + x + 1);
             if (x >= stride_px) past_end[r][at + x] = 1;
         }
     }
@@ -817,8 +820,9 @@ uint32_t wave_roots_setting() {
 
 namespace mrt_host {
 
+// attempt: 0, or how often the wavefront has overflowed its queues (see there)
 static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o, uint32_t *d_bitmap, uint32_t stride,
-                       float *d_accum, MrtRenderStats *stats, uint32_t strata, HostOut *out) {
+                       float *d_accum, MrtRenderStats *stats, uint32_t strata, HostOut *out, int attempt = 0) {
     MrtContext *ctx = s->ctx;
     cudaStream_t q = ctx->stream;
     const uint32_t stride_px = stride / 4u;
@@ -890,6 +894,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
     const int grid = ctx->sm_count * 16;
     uint64_t rays_closest = 0, rays_shadow = 0;
     bool counted = false;    // the kernels count the rays
+    bool again = false;      // what overflows is rendered again
     uint32_t launches = 0;   // kernels launched by this render
     float trace_ms = 0.0f;
     int trace_pairs = 0;   // recorded pairs of ctx->trace_ev not yet added to trace_ms
@@ -1021,7 +1026,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         if (!roots) {
             roots = kWaveRoots;
             const uint64_t need = 2ull * kWaveRoots * ((uint64_t)(levels + 2) * (kRayBytes + kNodeBytes) + std::max(1u, o->spl) * 2ull * kShadowBytes);
-            if (!paths && !ctx->arena && max_round * o->spp > kWaveRoots) {
+            if (!paths && !ctx->arena && attempt == 0 && max_round * o->spp > kWaveRoots) {
                 size_t free_bytes = 0, all_bytes = 0;
                 const bool held = ctx->wave[2].bytes >= 2ull * kWaveRoots * (uint64_t)(levels + 2) * kNodeBytes;   // allocated before
                 if (held || (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && need <= free_bytes / 8)) roots = 2u * kWaveRoots;
@@ -1031,13 +1036,22 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         // own stream and half of the queues: the tail of one wave's level (its longest rays, then a launch)
         // overlaps the other's bulk (terrain PathTracer 32.0 -> 31.1 ms, glass room 2.22 -> 2.0 to 2.19).
         // The folds stay in wave order.
+        // A wave's queues hold levels + 2 rays a path.  The two waves of a round that one pair takes are dealt its
+        // tasks in turn (wave_task) and need about the same.  Should one overflow all the same where the queues
+        // might hold the waves one by one, the frame is rendered again, from the caller's pixels and sums as
+        // they were, as single waves of up to 2^21 paths with all of the queues.  Frames of an explicit list
+        // with more paths than that, whose tasks come tile by tile, go on with waves of half the size each time.
         int pipes = 1;
+        bool pair = !paths && attempt == 0, deal = false;
+        const size_t keep_bitmap = (4 * plan.end + 255) & ~(size_t)255, keep_sums = d_accum ? 16ull * o->width * o->height : 0;
         uint32_t wave = 0;
         uint64_t ray_cap = 0, shadow_cap = 0;
         for (;;) {
             const uint32_t most = (uint32_t)std::min<uint64_t>(max_round * o->spp, paths ? std::max(roots, 1u << 22) : roots);
-            pipes = !paths && most >= kPairedRoots ? 2 : 1;
+            pipes = pair && most >= kPairedRoots ? 2 : 1;
             wave = (most + (uint32_t)pipes - 1u) / (uint32_t)pipes;
+            deal = pipes == 2 && most == max_round * o->spp && (uint64_t)kDealTasks * o->spp <= wave / 8u;
+            if (deal) wave += kDealTasks * o->spp;   // of the groups one wave may have one more, the other a part
             // (multiples of 4: the second wave's records start on 32 bytes)
             ray_cap = paths ? 0 : ((uint64_t)wave * (uint64_t)(levels + 2) + 3) & ~3ull;
             shadow_cap = paths ? 0 : ((uint64_t)wave * std::max(1u, o->spl) * 2ull + 3) & ~3ull;
@@ -1048,11 +1062,18 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], kNodeBytes * ray_cap * pipes);
                 if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], kShadowBytes * shadow_cap * pipes);
             }
-            if (st != MRT_ERR_OOM || roots <= kWaveRoots) break;
-            roots = kWaveRoots;   // no room for the large wave after all
-            for (int k = 1; k <= 3; ++k) dev_free(ctx->wave[k]);
+            if (st == MRT_OK && pipes == 2) st = ensure(ctx, ctx->wave[6], keep_bitmap + keep_sums);
+            if (st != MRT_ERR_OOM || (roots <= kWaveRoots && pipes == 1)) break;
+            if (roots > kWaveRoots) {   // no room for the large wave after all
+                roots = kWaveRoots;
+                for (int k = 1; k <= 3; ++k) dev_free(ctx->wave[k]);
+            } else {
+                pair = false;
+            }
             st = MRT_OK;
         }
+        again = pipes == 2 || (attempt > 0 && !plan.implicit && max_round * o->spp > roots && wave >> attempt >= 1024u);
+        if (attempt > 1) wave >>= attempt - 1;
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[4], sizeof(Level) * (levels + 2) * pipes);
         if (st == MRT_OK) st = ensure(ctx, ctx->wave[5], sizeof(float4) * (size_t)wave * pipes);
         if (st != MRT_OK) return st;
@@ -1070,6 +1091,15 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         }
         // the work counters of the first waves and the ray counters
         cudaMemsetAsync(ctx->d_counters, 0, MrtContext::kWorkCounters * sizeof(uint32_t) + 16, q);
+        if (pipes == 2 || attempt > 0) {   // keep the caller's pixels, or take them back
+            void *kept[2] = {ctx->wave[6].ptr, (char *)ctx->wave[6].ptr + keep_bitmap}, *own[2] = {d_bitmap, d_accum};
+            const size_t bytes[2] = {4 * plan.end, keep_sums};
+            for (int k = 0; k < 2 && st == MRT_OK; ++k)
+                if (bytes[k])
+                    st = cuda_status(ctx, cudaMemcpyAsync(attempt ? own[k] : kept[k], attempt ? kept[k] : own[k], bytes[k],
+                                                          cudaMemcpyDeviceToDevice, q), "pixels kept");
+            if (st != MRT_OK) return st;
+        }
         if (pipes == 2) {
             cudaEventRecord(ctx->fork_ev, q);
             cudaStreamWaitEvent(ctx->wave_stream, ctx->fork_ev, 0);
@@ -1081,7 +1111,11 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         for (size_t rd = 0; rd < plan.round_first.size(); ++rd) {
             p.task_base = plan.round_first[rd];
             const uint64_t total_roots = (uint64_t)plan.round_count[rd] * o->spp;
-            for (uint64_t r0 = 0; r0 < total_roots; r0 += wave) {
+            const bool dealt = deal && total_roots > wave;
+            const uint64_t group = (uint64_t)kDealTasks * o->spp, groups = total_roots / group;
+            // the even groups' paths: half of the pairs of groups, and of what follows them at most one group
+            const uint64_t even = groups / 2 * group + std::min(group, total_roots - groups / 2 * 2 * group);
+            for (uint64_t r0 = 0, step; r0 < total_roots; r0 += step) {
                 if (waves_issued >= 2) {
                     const int slot = (int)(waves_issued % 2);
                     st = cuda_status(ctx, cudaEventSynchronize(ctx->wave_ev[slot]), "render");
@@ -1093,8 +1127,10 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
                 WaveState &w = pipe[k];
                 cudaStream_t wq = k ? ctx->wave_stream : q;
                 uint32_t *work = ctx->d_counters + k * MrtContext::kWaveCounters;
-                w.root_first = (uint32_t)r0;
-                w.n_roots = (uint32_t)std::min<uint64_t>(wave, total_roots - r0);
+                step = std::min<uint64_t>(dealt ? (r0 ? total_roots - even : even) : wave, total_roots - r0);
+                w.root_first = dealt ? 0u : (uint32_t)r0;
+                w.n_roots = (uint32_t)step;
+                w.deal = dealt ? (r0 ? 2u : 1u) : 0u;
                 if (paths) {
                     if (waves_issued) cudaMemsetAsync(ctx->d_counters, 0, sizeof(uint32_t), q);
                     const bool small = small_paths(o->shader, s->n_tri) &&
@@ -1136,11 +1172,19 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         rays_closest = ctx->status->count[0];
         rays_shadow = ctx->status->count[1];
     }
+    float ms = 0.0f;
+    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+    if (st == MRT_ERR_LIMIT && again) {
+        st = render_impl(s, cam, o, d_bitmap, stride, d_accum, stats, strata, out, attempt + 1);
+        if (stats && st == MRT_OK) {
+            stats->device_ms += ms;
+            stats->kernel_launches += launches;
+        }
+        return st;
+    }
     s->progress.store(o->spp);
     add_trace_time();
     if (stats) {
-        float ms = 0.0f;
-        cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
         stats->rays_closest = rays_closest;
         stats->rays_shadow = rays_shadow;
         stats->paths = (uint64_t)plan.n_tasks * o->spp;

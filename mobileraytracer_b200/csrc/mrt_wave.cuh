@@ -298,6 +298,7 @@ struct WaveState {
     float4 *root_rgb;        // per wave root: rgb, flag
     uint32_t root_first;     // global index of the wave's first root
     uint32_t n_roots;
+    uint32_t deal;           // 0: consecutive tasks; 1, 2: even and odd groups of kDealTasks tasks (wave_task)
     unsigned long long *counters;   // [0] closest rays, [1] shadow rays
     // per-material shade queues: the shade kernel sorts each window of a level's rays by shading
     // class before shading them (scenes that mix diffuse with mirror / glass materials)
@@ -340,15 +341,22 @@ __device__ __forceinline__ uint32_t warp_alloc(uint32_t want, uint32_t *counter)
     return base + incl - want;
 }
 
+// The round's task of a wave's task t.  Two waves that split a round take groups of it in turn: rays branch
+// unevenly over a frame, and a half of its rows could need more of the queues than the frame (glass_room() from
+// inside, depth_max 4: 6.2 rays a path, 7.6 in the upper half, of 7 that the queues hold).
+constexpr uint32_t kDealTasks = 64;
+__device__ __forceinline__ uint32_t wave_task(const WaveState &w, uint32_t t) {
+    return w.deal ? (2u * (t / kDealTasks) + (w.deal - 1u)) * kDealTasks + t % kDealTasks : t;
+}
+
 __device__ __forceinline__ void root_task(const RenderParams &p, const WaveState &w, uint32_t root, Task &k,
                                           uint32_t &pixel, uint32_t &sample) {
     const uint32_t g = w.root_first + root;
-    const uint32_t t = p.task_base + g / p.spp, si = g % p.spp;
+    const uint32_t t = p.task_base + wave_task(w, g / p.spp), si = g % p.spp;
     k = task_of(p, t);
     pixel = k.y * p.width + k.x;
     sample = p.spp_offset + si;
 }
-
 
 __device__ __forceinline__ Ray ray_of(const RayRec &r) {
     Ray x;
