@@ -194,7 +194,7 @@ void dev_free(DevBuf &b) {
 
 int ensure(MrtContext *ctx, DevBuf &b, size_t bytes) {
     if (b.ptr && b.bytes >= bytes) return MRT_OK;
-    return dev_alloc(ctx, b, bytes + bytes / 4);
+    return dev_alloc(ctx, b, grown(bytes));
 }
 
 int check_kernel_error(MrtContext *ctx) {

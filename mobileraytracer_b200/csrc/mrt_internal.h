@@ -119,7 +119,8 @@ bool set_error(MrtContext *ctx, const char *fmt, ...);
 int cuda_status(MrtContext *ctx, cudaError_t e, const char *what);
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes);
 void dev_free(DevBuf &b);
-int ensure(MrtContext *ctx, DevBuf &b, size_t bytes);   // grow-only scratch
+inline size_t grown(size_t bytes) { return bytes + bytes / 4; }
+int ensure(MrtContext *ctx, DevBuf &b, size_t bytes);   // grow-only scratch: a larger buffer takes grown(bytes)
 void drain(MrtContext *ctx);                            // waits for all work of the context's streams
 void drain(MrtScene *s);                                // and for batches with jobs on the scene
 int check_kernel_error(MrtContext *ctx);                // waits for the stream, reads and clears the error flag

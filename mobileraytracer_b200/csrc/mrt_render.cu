@@ -801,10 +801,10 @@ uint64_t paths_max_setting() {
 
 constexpr uint32_t kPairedRoots = 1u << 19;   // paths from which a wavefront runs as two waves at once
 
-// Paths in flight of a wavefront render: 2^22 where their queues (7 GB at depth 6) take at most an eighth of
-// the free device memory, 2^21 otherwise and on an arena, whose owner has sized it (MRT_WAVE_ROOTS: that
+// Paths in flight of a wavefront render: 2^22 where their queues (9.1 GB at depth 6, a quarter of it room to
+// grow) take at most an eighth of the memory that is free without them, 2^21 otherwise and on an arena, whose owner has sized it (MRT_WAVE_ROOTS: that
 // many).  Larger waves pay fewer tails and launches: the 1024x1024x16 terrain PathTracer takes 39.1 ms at
-// 2^20, 31.2 at 2^21, 27.3 at 2^22, 25.8 at 2^23 (14 GB, whose first allocation costs more than it gives).
+// 2^20, 31.2 at 2^21, 27.3 at 2^22, 25.8 at 2^23 (18 GB, whose first allocation costs more than it gives).
 constexpr uint32_t kWaveRoots = 1u << 21;
 uint32_t wave_roots_setting() {
     static uint32_t v = [] {
@@ -1022,16 +1022,6 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         uint64_t max_round = 0;
         for (uint32_t c : plan.round_count) max_round = std::max<uint64_t>(max_round, c);
         const int levels = std::max(1, o->depth_max + 1);
-        uint32_t roots = wave_roots_setting();
-        if (!roots) {
-            roots = kWaveRoots;
-            const uint64_t need = 2ull * kWaveRoots * ((uint64_t)(levels + 2) * (kRayBytes + kNodeBytes) + std::max(1u, o->spl) * 2ull * kShadowBytes);
-            if (!paths && !ctx->arena && attempt == 0 && max_round * o->spp > kWaveRoots) {
-                size_t free_bytes = 0, all_bytes = 0;
-                const bool held = ctx->wave[2].bytes >= 2ull * kWaveRoots * (uint64_t)(levels + 2) * kNodeBytes;   // allocated before
-                if (held || (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && need <= free_bytes / 8)) roots = 2u * kWaveRoots;
-            }
-        }
         // Wavefronts of at least kPairedRoots paths run as two waves of half the size at once, each on its
         // own stream and half of the queues: the tail of one wave's level (its longest rays, then a launch)
         // overlaps the other's bulk (terrain PathTracer 32.0 -> 31.1 ms, glass room 2.22 -> 2.0 to 2.19).
@@ -1046,7 +1036,8 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         const size_t keep_bitmap = (4 * plan.end + 255) & ~(size_t)255, keep_sums = d_accum ? 16ull * o->width * o->height : 0;
         uint32_t wave = 0;
         uint64_t ray_cap = 0, shadow_cap = 0;
-        for (;;) {
+        size_t queue_bytes[3] = {0, 0, 0};   // of ctx->wave[1 .. 3]
+        auto size_waves = [&](uint32_t roots) {
             const uint32_t most = (uint32_t)std::min<uint64_t>(max_round * o->spp, paths ? std::max(roots, 1u << 22) : roots);
             pipes = pair && most >= kPairedRoots ? 2 : 1;
             wave = (most + (uint32_t)pipes - 1u) / (uint32_t)pipes;
@@ -1055,12 +1046,31 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
             // (multiples of 4: the second wave's records start on 32 bytes)
             ray_cap = paths ? 0 : ((uint64_t)wave * (uint64_t)(levels + 2) + 3) & ~3ull;
             shadow_cap = paths ? 0 : ((uint64_t)wave * std::max(1u, o->spl) * 2ull + 3) & ~3ull;
+            queue_bytes[0] = kRayBytes * ray_cap * pipes;
+            queue_bytes[1] = kNodeBytes * ray_cap * pipes;
+            queue_bytes[2] = kShadowBytes * shadow_cap * pipes;
+        };
+        uint32_t roots = wave_roots_setting();
+        if (!roots) {
+            roots = kWaveRoots;
+            if (!paths && !ctx->arena && attempt == 0 && max_round * o->spp > kWaveRoots) {
+                size_waves(2u * kWaveRoots);
+                size_t now = 0, then = 0, free_bytes = 0, all_bytes = 0;   // what the three buffers take
+                for (int k = 0; k < 3; ++k) {
+                    const size_t held = ctx->wave[1 + k].bytes;
+                    now += held;
+                    then += held >= queue_bytes[k] ? held : grown(queue_bytes[k]);
+                }
+                if (then == now || (cudaMemGetInfo(&free_bytes, &all_bytes) == cudaSuccess && then <= (free_bytes + now) / 8))
+                    roots = 2u * kWaveRoots;
+            }
+        }
+        for (;;) {
+            size_waves(roots);
             if (ray_cap * pipes > 0xFFFFFFF0ull) { set_error(ctx, "mrt_render: wave too large"); return MRT_ERR_ARG; }
             if (2 * (levels + 1) > MrtContext::kWaveCounters) { set_error(ctx, "mrt_render: depth_max above 30"); return MRT_ERR_ARG; }
             if (!paths) {   // the wavefront's queues (whole-path launches keep their state per lane)
-                st = ensure(ctx, ctx->wave[1], kRayBytes * ray_cap * pipes);
-                if (st == MRT_OK) st = ensure(ctx, ctx->wave[2], kNodeBytes * ray_cap * pipes);
-                if (st == MRT_OK) st = ensure(ctx, ctx->wave[3], kShadowBytes * shadow_cap * pipes);
+                for (int k = 0; k < 3 && st == MRT_OK; ++k) st = ensure(ctx, ctx->wave[1 + k], queue_bytes[k]);
             }
             if (st == MRT_OK && pipes == 2) st = ensure(ctx, ctx->wave[6], keep_bitmap + keep_sums);
             if (st != MRT_ERR_OOM || (roots <= kWaveRoots && pipes == 1)) break;
