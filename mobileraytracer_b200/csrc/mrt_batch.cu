@@ -787,6 +787,7 @@ void free_batch(MrtBatch *b) {
     dev_free(b->d_jobs);
     dev_free(b->d_scenes);
     dev_free(b->d_counters);
+    trim_pool(b->ctx);
     if (b->h_jobs) cudaFreeHost(b->h_jobs);
     if (b->h_scenes) cudaFreeHost(b->h_scenes);
     if (b->h_desc) cudaFreeHost(b->h_desc);

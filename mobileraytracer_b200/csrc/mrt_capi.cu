@@ -81,17 +81,13 @@ static void arena_free(MrtArena *a, void *p, size_t bytes) {
 // made with the first of them.  Opening a scene allocates and frees some 45 buffers; with cudaMalloc and
 // cudaFree, each of which maps memory and waits for the device, a 200,003-triangle scene took 16 to 57 ms
 // to upload, build and render once, of which the kernels are 0.9 ms.  The pool keeps at most kPoolKeep
-// unused bytes (trim_pool, after builds and when scenes go) and none once the device's last context is
-// gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight.  For a pooled
-// buffer cudaFree does not wait, and another context may be given the memory at once, so whoever frees waits
-// first (drain): calls that end in an error with work queued, a buffer replaced by a larger one, a scene destroyed
-// or built again.  Larger buffers are few and long-lived (ray pools) and would only make the
+// unused bytes (trim_pool, at the end of each call that frees buffers) and none once the device's last
+// context is gone.  A buffer is freed like any other, by cudaFree: when no work that uses it is in flight.
+// For a pooled buffer cudaFree does not wait, and another context may be given the memory at once, so whoever
+// frees waits first (drain): calls that end in an error with work queued, a buffer replaced by a larger one, a
+// scene destroyed or built again.  Larger buffers are few and long-lived (ray pools) and would only make the
 // pool's bound meaningless.
 constexpr size_t kPoolMost = 256u << 20, kPoolKeep = 1u << 30;
-struct DevicePool {
-    cudaMemPool_t pool = nullptr;
-    int contexts = 0;
-};
 std::mutex g_pool_mu;
 std::map<int, DevicePool> g_pools;
 
@@ -109,23 +105,23 @@ int pool_join(MrtContext *ctx) {
         uint64_t keep = ~0ull;   // nothing is given back by itself: trim_pool bounds what is unused
         cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep);
     }
-    ctx->pool = d.pool;
+    ctx->pool = &d;
     ++d.contexts;
     return MRT_OK;
+}
+// (cudaMemPoolAttrUsedMemCurrent does not go down when a buffer is freed by cudaFree)
+void trim_pool(MrtContext *ctx) {
+    uint64_t reserved = 0;
+    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess) return;
+    const uint64_t most = ctx->pool->used.load() + kPoolKeep;
+    if (reserved > most) cudaMemPoolTrimTo(ctx->pool->pool, (size_t)most);
 }
 void pool_leave(MrtContext *ctx) {
     if (!ctx->pool) return;
     std::lock_guard<std::mutex> lock(g_pool_mu);
-    DevicePool &d = g_pools[ctx->device];
-    if (--d.contexts == 0) cudaMemPoolTrimTo(d.pool, 0);
+    if (--ctx->pool->contexts == 0) cudaMemPoolTrimTo(ctx->pool->pool, 0);
+    else trim_pool(ctx);
     ctx->pool = nullptr;
-}
-void trim_pool(MrtContext *ctx) {
-    uint64_t reserved = 0, used = 0;
-    if (!ctx->pool || cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
-        cudaMemPoolGetAttribute(ctx->pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess)
-        return;
-    if (reserved - used > kPoolKeep) cudaMemPoolTrimTo(ctx->pool, (size_t)used + kPoolKeep);
 }
 
 void drain(MrtContext *ctx) {
@@ -139,8 +135,11 @@ void drain(MrtScene *s) {
 }
 
 int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
-    if (b.ptr) drain(ctx);
-    dev_free(b);
+    if (b.ptr) {
+        drain(ctx);
+        dev_free(b);
+        trim_pool(ctx);
+    }
     if (bytes == 0) bytes = 16;
     if (ctx->arena) {
         b.ptr = arena_alloc(ctx->arena, bytes);
@@ -160,16 +159,19 @@ int dev_alloc(MrtContext *ctx, DevBuf &b, size_t bytes) {
     }
     cudaError_t e = cudaErrorMemoryAllocation;
     if (ctx->pool && bytes < kPoolMost) {
-        e = cudaMallocFromPoolAsync(&b.ptr, bytes, ctx->pool, ctx->stream);
-        if (e != cudaSuccess) {
+        e = cudaMallocFromPoolAsync(&b.ptr, bytes, ctx->pool->pool, ctx->stream);
+        if (e == cudaSuccess) {
+            b.pool = ctx->pool;
+            b.pool->used += bytes;
+        } else {
             cudaGetLastError();
-            cudaMemPoolTrimTo(ctx->pool, 0);
+            cudaMemPoolTrimTo(ctx->pool->pool, 0);
         }
     }
     if (e != cudaSuccess) e = cudaMalloc(&b.ptr, bytes);
     if (e == cudaErrorMemoryAllocation && ctx->pool) {   // what the pool keeps unused may be what is missing
         cudaGetLastError();
-        cudaMemPoolTrimTo(ctx->pool, 0);
+        cudaMemPoolTrimTo(ctx->pool->pool, 0);
         e = cudaMalloc(&b.ptr, bytes);
     }
     if (e != cudaSuccess) {
@@ -188,8 +190,10 @@ void dev_free(DevBuf &b) {
         else cudaFree(b.ptr);
     }
     b.ptr = nullptr;
+    if (b.pool) b.pool->used -= b.bytes;
     b.bytes = 0;
     b.arena = nullptr;
+    b.pool = nullptr;
 }
 
 int ensure(MrtContext *ctx, DevBuf &b, size_t bytes) {
@@ -549,6 +553,7 @@ int mrt_scene_create(MrtContext *ctx, const MrtSceneDesc *d, MrtScene **out) {
     dev_free(st_abc); dev_free(st_n); dev_free(st_c); dev_free(st_m);
     if (st != MRT_OK) {
         scene_free(s);
+        trim_pool(ctx);
         delete s;
         return st;
     }
@@ -614,8 +619,8 @@ int mrt_scene_build(MrtScene *s, const MrtAccelOpts *o) {
         if (o->camera) camera_box(*o->camera, cmn, cmx);
         st = build_grids(s, cmn, cmx, o->grid_size, o->grid_index);
     }
-    if (st != MRT_OK) { drain(ctx); return st; }
-    st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_scene_build");
+    if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_scene_build");
+    else drain(ctx);
     trim_pool(ctx);
     if (st == MRT_OK) s->built = true;
     return st;

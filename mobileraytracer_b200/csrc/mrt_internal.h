@@ -16,11 +16,20 @@
 #include "mrt_device.cuh"
 
 struct MrtArena;
+struct DevicePool;
 
 struct DevBuf {
     void *ptr = nullptr;
     size_t bytes = 0;
-    MrtArena *arena = nullptr;   // carved from this arena (nullptr: cudaMalloc)
+    MrtArena *arena = nullptr;    // carved from this arena,
+    DevicePool *pool = nullptr;   // from this pool (neither: cudaMalloc)
+};
+
+// The memory pool of a device's contexts (mrt_capi.cu).
+struct DevicePool {
+    cudaMemPool_t pool = nullptr;
+    int contexts = 0;
+    std::atomic<uint64_t> used{0};   // bytes of the buffers from it
 };
 
 // One device allocation carved into the buffers of many scenes (geometry, trees, build scratch):
@@ -55,7 +64,7 @@ struct MrtContext {
     static constexpr int kWaveCounters = 64;       // of one wave
     static constexpr int kWorkCounters = 2 * kWaveCounters;
     unsigned long long *ray_counters() const { return reinterpret_cast<unsigned long long *>(d_counters + kWorkCounters); }
-    cudaMemPool_t pool = nullptr;       // the device's pool (mrt_capi.cu)
+    DevicePool *pool = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     static constexpr int kTraceEvents = 16;             // start / end pairs around traversal launches
     cudaEvent_t trace_ev[2 * kTraceEvents] = {};

@@ -1077,6 +1077,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
             if (roots > kWaveRoots) {   // no room for the large wave after all
                 roots = kWaveRoots;
                 for (int k = 1; k <= 3; ++k) dev_free(ctx->wave[k]);
+                trim_pool(ctx);
             } else {
                 pair = false;
             }

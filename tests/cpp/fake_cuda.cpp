@@ -26,6 +26,7 @@ struct Event {
 
 std::set<Stream *> g_streams;
 std::map<void *, std::pair<size_t, bool>> g_live;   // device memory: bytes, of a pool
+uint64_t g_pool_allocated = 0;
 cudaError_t g_last = cudaSuccess;
 
 void finish(Stream *s, uint64_t at) {
@@ -62,6 +63,11 @@ uint64_t allocations = 0, operations = 0, launches = 0, violations = 0, failed =
 uint64_t fail_allocations_from = ~0ull, fail_operations_from = ~0ull;
 uint64_t pool_reserved = 0;
 void (*on_copy_out)(void *dst, size_t bytes) = nullptr;
+uint64_t pool_used() {
+    uint64_t n = 0;
+    for (auto &b : g_live) n += b.second.second ? b.second.first : 0;
+    return n;
+}
 size_t live_buffers() { return g_live.size(); }
 void reset() {
     finish_all();
@@ -71,12 +77,6 @@ void reset() {
     g_last = cudaSuccess;
 }
 }  // namespace fake
-
-static size_t pool_used() {
-    size_t n = 0;
-    for (auto &b : g_live) n += b.second.second ? b.second.first : 0;
-    return n;
-}
 
 extern "C" {
 
@@ -94,7 +94,8 @@ cudaError_t cudaMemGetInfo(size_t *free_bytes, size_t *total) { *free_bytes = *t
 cudaError_t cudaMalloc(void **p, size_t bytes) { return allocate(p, bytes, false); }
 cudaError_t cudaMallocFromPoolAsync(void **p, size_t bytes, cudaMemPool_t, cudaStream_t) {
     const cudaError_t e = allocate(p, bytes, true);
-    if (pool_used() > fake::pool_reserved) fake::pool_reserved = pool_used();
+    if (e == cudaSuccess) g_pool_allocated += bytes;
+    if (fake::pool_used() > fake::pool_reserved) fake::pool_reserved = fake::pool_used();
     return e;
 }
 cudaError_t cudaFree(void *p) {
@@ -115,12 +116,13 @@ cudaError_t cudaMemPoolCreate(cudaMemPool_t *pool, const cudaMemPoolProps *) {
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolSetAttribute(cudaMemPool_t, enum cudaMemPoolAttr, void *) { return cudaSuccess; }
+// (the used bytes that the runtime reports do not go down with cudaFree; cudaFreeAsync is not modelled)
 cudaError_t cudaMemPoolGetAttribute(cudaMemPool_t, enum cudaMemPoolAttr a, void *v) {
-    *static_cast<uint64_t *>(v) = a == cudaMemPoolAttrReservedMemCurrent ? fake::pool_reserved : pool_used();
+    *static_cast<uint64_t *>(v) = a == cudaMemPoolAttrReservedMemCurrent ? fake::pool_reserved : g_pool_allocated;
     return cudaSuccess;
 }
 cudaError_t cudaMemPoolTrimTo(cudaMemPool_t, size_t keep) {
-    if (fake::pool_reserved > keep) fake::pool_reserved = keep > pool_used() ? keep : pool_used();
+    if (fake::pool_reserved > keep) fake::pool_reserved = keep > fake::pool_used() ? keep : fake::pool_used();
     return cudaSuccess;
 }
 

@@ -10,6 +10,7 @@ extern uint64_t failed;                              // operations and allocatio
 extern uint64_t fail_allocations_from, fail_operations_from;
 extern uint64_t pool_reserved;                       // bytes the pool holds, in use or not
 extern void (*on_copy_out)(void *dst, size_t bytes); // after a device-to-host copy
+uint64_t pool_used();                                 // of these
 size_t live_buffers();
 void reset();                                        // counts and failures; queued work is done
 }

@@ -43,3 +43,7 @@ def test_scene_creation_and_builds_that_fail(objects):
 
 def test_scenes_that_go_while_a_batch_reads_them(objects):
     _run(objects, "scene_in_use")
+
+
+def test_the_pool_keeps_at_most_a_gibibyte(objects):
+    _run(objects, "pool_bound")
