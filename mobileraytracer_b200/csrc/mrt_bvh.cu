@@ -5,9 +5,9 @@
 // reorders primitives, so leaf offsets index the input arrays.
 //
 // FAST tree: built on the device.  Triangle boxes padded outward -> 30-bit Morton codes of the
-// centroids on a grid of cubes -> stable LSD radix sort (own kernels) -> Karras' parallel hierarchy
-// ("Maximizing parallelism in the construction of BVHs, octrees and k-d trees", HPG 2012) -> bottom-up
-// box fit, which also works out for every binary node the cheapest way to turn its subtree into wide
+// centroids, cells halved along their longest side -> stable LSD radix sort (own kernels) -> Karras'
+// parallel hierarchy ("Maximizing parallelism in the construction of BVHs, octrees and k-d trees", HPG
+// 2012) -> bottom-up box fit, which also works out for every binary node the cheapest way to turn its subtree into wide
 // nodes -> the binary tree collapsed along those choices into 8-wide nodes with 16-bit quantised
 // child boxes (128 bytes: one cache line per traversal step), children placed in slots by octant,
 // internal children numbered consecutively, the leaf children's triangles copied to consecutive
@@ -148,37 +148,58 @@ __global__ void k_tri_boxes(uint32_t n, const float4 *__restrict__ a4, const flo
     }
 }
 
-__device__ __forceinline__ uint32_t expand_bits(uint32_t v) {   // 10 bits -> every third bit
-    v = (v * 0x00010001u) & 0xFF0000FFu;
-    v = (v * 0x00000101u) & 0x0F00F00Fu;
-    v = (v * 0x00000011u) & 0xC30C30C3u;
-    v = (v * 0x00000005u) & 0x49249249u;
-    return v;
-}
-
-// Codes on a grid of cubes over the longest side of the centroid bounds, 1024 a side.  (A grid of
-// 1024 cells along every axis whatever its extent cuts flat scenes across their thin axis as often as
-// along the others: on the 524,288-triangle heightfield, 0.35 high over a side of 2, a camera ray then
-// visits 10.9 nodes and a bounce 16.4, with cubes 9.1 and 14.4; scenes as deep as wide keep their codes.)
-__global__ void k_morton(uint32_t n, const float4 *__restrict__ bmin, const float4 *__restrict__ bmax,
-                         const uint32_t *__restrict__ cbounds, uint32_t *keys, uint32_t *vals) {
+// 30 bits along the three axes of the centroid bounds: each halves the cells along their longest side, an axis at
+// most 13 times.  Sides are compared by their octave (equal ones: x, y, z in turn): by their lengths, a soup whose
+// bounds are a thousandth off a cube gets another order of the axes, and its 1080p frame took 1,135 us, not 1,112.
+// Ten bits an axis in turn, whatever the sides, cut flat scenes across their thin axis as often as along the
+// others; cubes of a 1024th of the longest side leave a model with one far triangle beside it a handful of cells.
+// Surface-area cost of the binary tree of 300,000 triangles against ten bits an axis in turn: sides 1 : 0.2 : 1
+// 0.78 (cubes 0.78), 100 : 1 : 1 0.30 (0.31), a cube of side 2 and one triangle 30, 200, 1,000 and 10^6 away 0.63,
+// 0.33, 0.21 and 1.00 (0.65, 1.61, 19.9, 84.6).  At most 10, 12 or 14 bits an axis: 0.58, 0.26 and 0.20 at 1,000,
+// 1.00, 1.00 and 1.01 at 10^6.  Nodes that a random ray visits in a soup of 1,000,000 alone 49, with a triangle
+// 200, 1,000 and 10^4 away 53, 58 and 177 (472, 16,163 and 100,530 with cubes, 149, 291 and 315 with ten bits in
+// turn); in the 524,288-triangle heightfield 6.2 (6.3, 7.2).
+constexpr int kCodeBits = 30, kAxisBits = 13;
+__global__ void __launch_bounds__(256) k_morton(uint32_t n, const float4 *__restrict__ bmin, const float4 *__restrict__ bmax,
+                                                const uint32_t *__restrict__ cbounds, uint32_t *keys, uint32_t *vals) {
+    __shared__ uint8_t axis_of[3 * kAxisBits];   // by place from the top bit
+    float mn[3], ext[3];
+    for (int k = 0; k < 3; ++k) {
+        mn[k] = key_float_(cbounds[k]);
+        ext[k] = key_float_(cbounds[3 + k]) - mn[k];
+        if (!(ext[k] > 0.0f && ext[k] <= 3.0e38f)) ext[k] = 0.0f;   // finite sides only
+    }
+    if (threadIdx.x < 3 * kAxisBits) {   // halving h of axis a goes behind those of longer cells
+        const float side = fmaxf(ext[0], fmaxf(ext[1], ext[2]));
+        int octave[3];
+        for (int k = 0; k < 3; ++k) octave[k] = ext[k] > 0.0f ? (int)rintf(log2f(side / ext[k])) : 1024;
+        const int a = threadIdx.x / kAxisBits, h = threadIdx.x % kAxisBits, own = octave[a] + h;
+        int place = 0;
+        for (int k = 0; k < 3; ++k)   // halvings j of axis k with octave[k] + j below own, or equal and k below a
+            place += min(max(own - octave[k] + (k < a ? 1 : 0), 0), kAxisBits);
+        axis_of[place] = (uint8_t)a;
+    }
+    __syncthreads();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 lo = bmin[i], hi = bmax[i];
     const float c[3] = {0.5f * (lo.x + hi.x), 0.5f * (lo.y + hi.y), 0.5f * (lo.z + hi.z)};
-    float mn[3], ext[3], side = 0.0f;
+    uint32_t q[3];   // the place along an axis, top bit first
     for (int k = 0; k < 3; ++k) {
-        mn[k] = key_float_(cbounds[k]);
-        ext[k] = key_float_(cbounds[3 + k]) - mn[k];
-        if (ext[k] > side && ext[k] <= 3.0e38f) side = ext[k];   // finite sides only
-    }
-    uint32_t q[3];
-    for (int k = 0; k < 3; ++k) {
-        float u = (ext[k] > 0.0f && ext[k] <= 3.0e38f) ? (c[k] - mn[k]) / side : 0.5f;
+        float u = ext[k] > 0.0f ? (c[k] - mn[k]) / ext[k] : 0.5f;
         u = fminf(fmaxf(u, 0.0f), 1.0f);
-        q[k] = min((uint32_t)(u * 1024.0f), 1023u);
+        q[k] = min((uint32_t)(u * (float)(1 << kAxisBits)), (1u << kAxisBits) - 1u) << (32 - kAxisBits);
     }
-    keys[i] = (expand_bits(q[0]) << 2) | (expand_bits(q[1]) << 1) | expand_bits(q[2]);
+    uint32_t code = 0;
+    for (int b = 0; b < kCodeBits; ++b) {
+        const int a = axis_of[b];
+        const uint32_t v = a == 0 ? q[0] : a == 1 ? q[1] : q[2];
+        code = code << 1 | v >> 31;
+        if (a == 0) q[0] <<= 1;
+        else if (a == 1) q[1] <<= 1;
+        else q[2] <<= 1;
+    }
+    keys[i] = code;
     vals[i] = i;
 }
 
@@ -690,7 +711,7 @@ int build_fast_bvh(MrtScene *s) {
                                       (float4 *)bmax.ptr, (uint32_t *)cb.ptr);
         k_morton<<<g, 256, 0, q>>>(n, (const float4 *)bmin.ptr, (const float4 *)bmax.ptr, (const uint32_t *)cb.ptr,
                                    (uint32_t *)keys[0].ptr, (uint32_t *)vals[0].ptr);
-        for (int shift = 0; shift < 30; shift += 8) {
+        for (int shift = 0; shift < kCodeBits; shift += 8) {
             k_rs_hist<<<nblocks, kSortThreads, 0, q>>>((const uint32_t *)keys[cur].ptr, n, shift, (uint32_t *)hist.ptr, nblocks);
             k_rs_scan_rows<<<256, 256, 0, q>>>((uint32_t *)hist.ptr, nblocks, (uint32_t *)total.ptr);
             k_rs_scatter<<<nblocks, kSortThreads, 0, q>>>((const uint32_t *)keys[cur].ptr, (const uint32_t *)vals[cur].ptr,

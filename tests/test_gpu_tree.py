@@ -1,7 +1,7 @@
 """The FAST tree at the sizes and shapes its build can go wrong at, against the oracle's exact closest hit and
 occlusion (GPU): one to a few triangles (root leaves of 1 to 3, a node that is not full), counts around a
 sort tile, triangles that coincide (no area to choose by, equal Morton codes), scenes along a line and in a
-plane (one or two axes without extent), far from the origin and of very different extents."""
+plane (one or two axes without extent), far from the origin and of very different extents.  A triangle far away costs the others' tree little."""
 import numpy as np
 import pytest
 
@@ -48,3 +48,25 @@ def test_tree_equals_every_triangle(ctx, kind, n):
     assert (g.trace_any(rays, dist) == o.trace_any(rays, dist)).all()
     assert 1 <= g.accel_info()["nodes"] <= max(1, n)
     g.close()
+
+
+def _nodes(ctx, sc, rays):
+    g = Scene(ctx, sc).build(capi.MRT_ACCEL_BVH, capi.MRT_BVH_FAST)
+    nodes = g.trace_counts(rays)[0].mean()
+    g.close()
+    return nodes
+
+
+# nodes a ray against the same scene without the far triangle (30.2): 30.6, 31.0, 31.1, 31.5 and 59.1 (92.7 with ten
+# bits of the code an axis in turn)
+@pytest.mark.parametrize("axis", [0, 1, 2])
+@pytest.mark.parametrize("far,most", [(4.0, 1.1), (30.0, 1.1), (200.0, 1.1), (1000.0, 1.2), (1e4, 2.5)])
+def test_a_far_triangle_costs_little(ctx, axis, far, most):
+    sc = scenes.triangle_soup(100_000, 5, 64, 64)
+    rays = random_rays(20_000, seed=9)
+    alone = _nodes(ctx, sc, rays)
+    away = sc.tri_abc[:1].copy().reshape(3, 3)
+    away[:, axis] += np.float32(far)
+    sc.tri_abc = np.concatenate([sc.tri_abc, away.reshape(1, 9)])
+    sc.tri_material = np.concatenate([sc.tri_material, sc.tri_material[:1]])
+    assert _nodes(ctx, sc, rays) <= most * alone + 1.0
