@@ -100,14 +100,6 @@ constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;
 
-__device__ __forceinline__ uint32_t float_key(float f) {   // order-preserving float -> uint
-    const uint32_t b = __float_as_uint(f);
-    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__device__ __forceinline__ float key_float_(uint32_t k) {
-    return __uint_as_float((k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k);
-}
-
 // padded triangle boxes (min.xyz, max.xyz as two float4) and the centroid bounds
 __global__ void k_tri_boxes(uint32_t n, const float4 *__restrict__ a4, const float4 *__restrict__ ab4,
                             const float4 *__restrict__ ac4, float4 *bmin, float4 *bmax, uint32_t *cbounds) {
@@ -131,7 +123,7 @@ __global__ void k_tri_boxes(uint32_t n, const float4 *__restrict__ a4, const flo
     }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (int k = 0; k < 3; ++k) {
-        uint32_t lo = valid ? float_key(c[k]) : 0xFFFFFFFFu, hi = valid ? float_key(c[k]) : 0u;
+        uint32_t lo = valid ? float_order(c[k]) : 0xFFFFFFFFu, hi = valid ? float_order(c[k]) : 0u;
         for (int o = 16; o > 0; o >>= 1) {
             lo = min(lo, __shfl_xor_sync(0xFFFFFFFFu, lo, o));
             hi = max(hi, __shfl_xor_sync(0xFFFFFFFFu, hi, o));
@@ -165,8 +157,8 @@ __global__ void __launch_bounds__(256) k_morton(uint32_t n, const float4 *__rest
     __shared__ uint8_t axis_of[3 * kAxisBits];   // by place from the top bit
     float mn[3], ext[3];
     for (int k = 0; k < 3; ++k) {
-        mn[k] = key_float_(cbounds[k]);
-        ext[k] = key_float_(cbounds[3 + k]) - mn[k];
+        mn[k] = order_float(cbounds[k]);
+        ext[k] = order_float(cbounds[3 + k]) - mn[k];
         if (!(ext[k] > 0.0f && ext[k] <= 3.0e38f)) ext[k] = 0.0f;   // finite sides only
     }
     if (threadIdx.x < 3 * kAxisBits) {   // halving h of axis a goes behind those of longer cells

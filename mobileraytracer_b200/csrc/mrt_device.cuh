@@ -10,6 +10,7 @@
 #pragma once
 
 #include <cstdint>
+#include <cstring>
 #include <cuda_runtime.h>
 
 #include "../../include/mrt_cuda.h"
@@ -58,6 +59,17 @@ MRT_HD float smin(float a, float b) { return (b < a) ? b : a; }
 MRT_HD float smax(float a, float b) { return (a < b) ? b : a; }
 MRT_HD V3 vmin(V3 a, V3 b) { return V3{smin(a.x, b.x), smin(a.y, b.y), smin(a.z, b.z)}; }
 MRT_HD V3 vmax(V3 a, V3 b) { return V3{smax(a.x, b.x), smax(a.y, b.y), smax(a.z, b.z)}; }
+// order-preserving float <-> uint (for atomicMin / atomicMax)
+__device__ __forceinline__ uint32_t float_order(float f) {
+    const uint32_t b = __float_as_uint(f);
+    return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
+}
+MRT_HD float order_float(uint32_t k) {
+    const uint32_t b = (k & 0x80000000u) ? (k & 0x7FFFFFFFu) : ~k;
+    float f;
+    memcpy(&f, &b, 4);
+    return f;
+}
 MRT_HD bool any_pos(V3 a) { return a.x > 0.0f || a.y > 0.0f || a.z > 0.0f; }
 MRT_HD float comp(V3 v, int k) { return k == 0 ? v.x : (k == 1 ? v.y : v.z); }
 // glm::reflect(I, N) = I - (N * dot(N, I)) * 2

@@ -271,6 +271,31 @@ __global__ void k_skip_bits(int64_t ncell, int64_t sy, int64_t sz, const uint32_
     }
 }
 
+// the union of the triangles' boxes: bounds[0..2] least and [3..5] greatest coordinates (float_order), [6] set when
+// a box has a coordinate that is not a number
+__global__ void __launch_bounds__(256) k_tri_bounds(DevScene s, uint32_t n, uint32_t *bounds) {
+    uint32_t lo[3] = {~0u, ~0u, ~0u}, hi[3] = {0u, 0u, 0u};
+    bool odd = false;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const Box b = prim_box<kTriangle>(s, i);
+        for (int k = 0; k < 3; ++k) {
+            const float mn = comp(b.mn, k), mx = comp(b.mx, k);
+            odd = odd || !(mn <= mx);
+            lo[k] = min(lo[k], float_order(mn));
+            hi[k] = max(hi[k], float_order(mx));
+        }
+    }
+    for (int k = 0; k < 3; ++k) {
+        lo[k] = __reduce_min_sync(0xFFFFFFFFu, lo[k]);
+        hi[k] = __reduce_max_sync(0xFFFFFFFFu, hi[k]);
+        if ((threadIdx.x & 31) == 0) {
+            atomicMin(&bounds[k], lo[k]);
+            atomicMax(&bounds[3 + k], hi[k]);
+        }
+    }
+    if (odd) bounds[6] = 1u;
+}
+
 uint32_t bit_counter(uint32_t n) { uint32_t c = 0; while (n > 0) { ++c; n >>= 1; } return c; }   // Utils.cpp:26-33
 uint32_t round_up_pow2(uint32_t v) {   // Utils.cpp:15-24
     --v; v |= v >> 1u; v |= v >> 2u; v |= v >> 4u; v |= v >> 8u; v |= v >> 16u; ++v; return v;
@@ -345,13 +370,34 @@ namespace mrt_host {
 int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int grid_size, int grid_index) {
     MrtContext *ctx = s->ctx;
     cudaStream_t q = ctx->stream;
-    const int got = host_triangles(s);
-    if (got != MRT_OK) return got;
+    // the triangles' bounds on the device (48 MB of 1,000,000 triangles read back took 17 of a build's 25 ms); with
+    // coordinates that are not numbers the order of the comparisons counts, and they are made here
+    V3 tri_mn{0.0f, 0.0f, 0.0f}, tri_mx{0.0f, 0.0f, 0.0f};
+    bool by_triangle = false;
+    if (s->n_tri) {
+        uint32_t h[7] = {~0u, ~0u, ~0u, 0u, 0u, 0u, 0u}, *d = ctx->d_counters;   // (free between calls)
+        int st = cuda_status(ctx, cudaMemcpyAsync(d, h, sizeof(h), cudaMemcpyHostToDevice, q), "grid bounds");
+        if (st != MRT_OK) return st;
+        k_tri_bounds<<<std::min<uint32_t>((s->n_tri + 255) / 256, (uint32_t)ctx->sm_count * 8), 256, 0, q>>>(s->dev, s->n_tri, d);
+        st = cuda_status(ctx, cudaGetLastError(), "grid bounds");
+        if (st == MRT_OK) st = cuda_status(ctx, cudaMemcpyAsync(h, d, sizeof(h), cudaMemcpyDeviceToHost, q), "grid bounds");
+        if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(q), "grid bounds");
+        by_triangle = h[6] != 0;
+        if (st == MRT_OK && by_triangle) st = host_triangles(s);
+        if (st != MRT_OK) return st;
+        tri_mn = V3{order_float(h[0]), order_float(h[1]), order_float(h[2])};
+        tri_mx = V3{order_float(h[3]), order_float(h[4]), order_float(h[5])};
+    }
     for (int type = 0; type < 3; ++type) {
         const uint32_t n = type == kTriangle ? s->n_tri : (type == kSphere ? s->n_sph : s->n_pln);
         // Scene::getBounds (Scene.cpp:42-45) over the primitives, then the camera (Camera.cpp:39-44)
         V3 mn{kRayLengthMax, kRayLengthMax, kRayLengthMax}, mx{-kRayLengthMax, -kRayLengthMax, -kRayLengthMax};
-        for (uint32_t i = 0; i < n; ++i) {
+        const bool known = type == kTriangle && n > 0 && !by_triangle;
+        if (known) {
+            mn = vmin(tri_mn, mn);
+            mx = vmax(tri_mx, mx);
+        }
+        for (uint32_t i = 0; i < n && !known; ++i) {
             const HostBox b = host_prim_box(s, type, i);
             mn = vmin(b.mn, mn);
             mx = vmax(b.mx, mx);

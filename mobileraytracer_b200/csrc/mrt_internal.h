@@ -135,7 +135,7 @@ void drain(MrtScene *s);                                // and for batches with 
 int check_kernel_error(MrtContext *ctx);                // waits for the stream, reads and clears the error flag
 void trim_pool(MrtContext *ctx);                        // gives memory beyond the pool's bound back
 
-// the triangles' A, AB, AC as the device has them in s->h_tri (the reference tree and the grid bounds need them)
+// the triangles' A, AB, AC as the device has them in s->h_tri (the reference tree needs them)
 int host_triangles(MrtScene *s);
 
 // builds (mrt_bvh.cu, mrt_grid.cu)

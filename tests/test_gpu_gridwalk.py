@@ -2,7 +2,8 @@
 their short cuts could go wrong: long empty runs (records that skip ahead), cells that share references
 (skip bits), both addressing modes at sizes that are and are not powers of two, the smallest grids, rays
 that start outside, run along axes or cell borders or have no direction, and distances that are not
-numbers (coordinates near the ends of the float range)."""
+numbers (coordinates near the ends of the float range).  Grids of triangles with coordinates that are not
+numbers or infinite, whose bounds depend on the order of the triangles."""
 import numpy as np
 import pytest
 
@@ -61,6 +62,21 @@ def test_walks_equal_the_reference_walk(ctx, kind, scale, size, index):
 
 def test_walks_with_planes_and_spheres(ctx):
     sc, rays = scenes.glass_room(), _rays(1.0)
+    g = Scene(ctx, sc).build(capi.MRT_ACCEL_REGULAR_GRID)
+    o = O.OrcScene(sc, 1)
+    assert _same(g.trace_closest(rays), o.trace_closest(rays)).all()
+    dist = np.full(len(rays), 1.2, np.float32)
+    assert (g.trace_any(rays, dist) == o.trace_any(rays, dist)).all()
+
+
+@pytest.mark.parametrize("value", [np.nan, np.inf, -np.inf])
+@pytest.mark.parametrize("at", [0, 700, 1499, None])
+def test_bounds_with_coordinates_that_are_not_finite(ctx, value, at):
+    sc, rays = _scene("small", 1.0), _rays(1.0)
+    if at is None:
+        sc.tri_abc[::10, 4] = value
+    else:
+        sc.tri_abc[at, 0:3] = value
     g = Scene(ctx, sc).build(capi.MRT_ACCEL_REGULAR_GRID)
     o = O.OrcScene(sc, 1)
     assert _same(g.trace_closest(rays), o.trace_closest(rays)).all()
