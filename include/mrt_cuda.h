@@ -398,7 +398,7 @@ typedef struct MrtBatchStats {
     double busy_ms;          /* device time with waves in flight (completed waves) */
     uint32_t wave_roots;     /* the settings in use (after autotuning) */
     uint32_t block_threads;
-    uint32_t blocks_per_sm;
+    uint32_t blocks_per_sm;  /* with MRT_BATCH_KERNEL_PATHS those of the latest wave */
     uint32_t autotuned;      /* candidates the autotuner timed (0: fixed settings) */
     uint32_t pipelines;
     uint32_t kernel;         /* MRT_BATCH_KERNEL_* chosen for waves dominated by one job */

@@ -600,7 +600,6 @@ int run_wave(MrtBatch *b, const WaveDesc &d, int pipe, uint32_t threads, uint32_
     MrtContext *ctx = b->ctx;
     BatchPipe &P = b->pipes[pipe];
     cudaStream_t q = P.stream;
-    if (threads == 0) bps = path_blocks(b, d);
     if (P.jobs_seen != b->jobs_uploaded) {
         cudaStreamWaitEvent(q, b->ev_jobs, 0);
         P.jobs_seen = b->jobs_uploaded;
@@ -678,7 +677,7 @@ int autotune(MrtBatch *b) {
     const MrtBatchOpts &o = b->opts;
     std::vector<std::pair<uint32_t, uint32_t>> shapes;
     if (o.kernel == MRT_BATCH_KERNEL_PATHS) {
-        shapes.push_back({0u, 8u});
+        shapes.push_back({0u, (uint32_t)kPathBlocksPerSm});
     } else if (o.block_threads && o.blocks_per_sm) {
         shapes.push_back({o.block_threads, o.blocks_per_sm});
     } else {
@@ -722,7 +721,7 @@ int autotune(MrtBatch *b) {
         cudaEventRecord(e0, q);
         for (uint32_t p = 0; p < np && st == MRT_OK; ++p) {
             cudaStreamWaitEvent(b->pipes[p].stream, e0, 0);
-            st = run_wave(b, d, (int)p, t, bps, -1, -1);
+            st = run_wave(b, d, (int)p, t, t == 0 ? path_blocks(b, d) : bps, -1, -1);
             cudaEventRecord(ep[p], b->pipes[p].stream);
             cudaStreamWaitEvent(q, ep[p], 0);
         }
@@ -882,7 +881,6 @@ int mrt_batch_create(MrtContext *ctx, const MrtBatchOpts *opts, MrtBatch **out) 
     if (st == MRT_OK) st = cuda_status(ctx, cudaMemsetAsync(b->d_counters.ptr, 0, 4 * sizeof(unsigned long long), ctx->stream), "memset");
     // the pipelines' streams use the buffers: wait for their allocation on the context's stream
     if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_batch_create");
-    if (st == MRT_OK) st = cuda_status(ctx, cudaStreamSynchronize(ctx->stream), "mrt_batch_create");
     if (st != MRT_OK) { free_batch(b); return st; }
     *out = b;
     return MRT_OK;
@@ -1001,6 +999,8 @@ int mrt_batch_step(MrtBatch *b, uint32_t max_waves, uint32_t *launched) {
             threads = 0;
             ++b->waves_paths;
         }
+        if (threads == 0) bps = path_blocks(b, d);
+        if (b->block_threads == 0) b->blocks_per_sm = bps;   // (MRT_BATCH_KERNEL_PATHS: what the statistics tell)
         st = run_wave(b, d, pipe, threads, bps, r, w > b->waves_done ? (int)((w - 1) % kRing) : -1);
         if (st != MRT_OK) return st;
         b->paths += n;

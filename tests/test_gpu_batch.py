@@ -179,3 +179,19 @@ def test_batch_rejects(ctx):
     assert len(b.completed()) == 1
     assert bool((bms[0] == bms[2]).all()) and bool((bms[0] == bms[1]).all())
     b.close()
+
+
+@pytest.mark.parametrize("scene,jobs,blocks", [("cornell", 12, 8), ("cornell", 2, 5), ("soup", 12, 5)])
+def test_stats_tell_the_blocks_of_whole_path_waves(ctx, scene, jobs, blocks):
+    """8 per SM where every job is a PathTracer of few triangles and there is a path for every lane, else 5."""
+    torch = _torch()
+    sc = scenes.cornell_box() if scene == "cornell" else scenes.triangle_soup(2000, 3, 128, 128)
+    g = Scene(ctx, sc).build()
+    b = Batch(ctx, wave_roots=1 << 18, kernel=capi.MRT_BATCH_KERNEL_PATHS, pipelines=1)
+    bms = [torch.zeros(128 * 128, dtype=torch.int32, device="cuda") for _ in range(jobs)]
+    for bm in bms:
+        b.submit(g, sc.camera, capi.render_opts(shader=PT, width=128, height=128, spp=1, depth_max=4), bm)
+    b.run()
+    st = b.stats()
+    assert (st.kernel, st.block_threads, st.blocks_per_sm) == (capi.MRT_BATCH_KERNEL_PATHS, 0, blocks)
+    b.close()
