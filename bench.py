@@ -419,7 +419,7 @@ def soup_frame(dist, ctx, sc, args, accel: int, mode: int, grid_size: int = 0, g
     shade = {"name": "k_ns_shade (per pixel: hit record 8 + triangle record 48 + shading 76 per hit + bitmap 8)",
              "algorithmic_bytes_per_launch": 16 * len(rays_np) + (48 + 76) * n_hit, "ms": ms - trace_ms}
     if accel == capi.MRT_ACCEL_REGULAR_GRID:
-        # the traversal kernel: cells 8 (start[c], start[c + 1]) + per reference 4 (index) + 48 (A, AB, AC)
+        # the traversal kernel: cells 8 (the cell's record) + per reference 4 (index) + 48 (A, AB, AC)
         # + the 8-byte hit record written
         alg = 8 * len(rays_np) + 8 * n_nodes + 52 * n_tris
         counts = {"cells_per_ray": n_nodes / len(rays_np), "refs_per_ray": n_tris / len(rays_np),

@@ -23,7 +23,7 @@
 //   * Cell records.  An empty cell's record says how many steps further every cell is empty (up to
 //     kEmptyReach); those steps read nothing.
 // On the 1080p frame of the soup at G = 128 a camera ray steps through 152 cells, 134 of them empty, and
-// meets 159 references, 79 of which are left to test.  Bound by the lanes' differing walks (13.7 of 32
+// meets 159 references, 79 of which are left to test.  Bound by the lanes' differing walks (11.8 of 32
 // active) and the latency of the triangle records; 6.48 -> 3.51 ms a frame, the any-hit rays above
 // 0.93 -> 0.59 ms (one ray a thread before).
 #pragma once

@@ -85,10 +85,6 @@ struct MrtContext {
     DevBuf raster[5];
 };
 
-struct RefBvhHost {
-    std::vector<mrt::RefNode> nodes;
-};
-
 struct MrtScene {
     MrtContext *ctx = nullptr;
     mrt::DevScene dev{};

@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(128, kNsBlocksPerSm) k_render_noshadows_fast(D
     persistent_closest<false>(s, w, lane);
 }
 
-// the same work on the RegularGrid: the persistent grid walk (mrt_gridwalk.cuh), one cell per lane
-// and loop iteration
+// the same work on the RegularGrid: the persistent grid walk (mrt_gridwalk.cuh), whose lanes step until
+// most hold references and test until most hold none
 __global__ void __launch_bounds__(128, kGridBlocksPerSm) k_render_noshadows_grid(DevScene s, RenderParams p, uint32_t first,
                                                                uint32_t count, uint32_t *ctr, uint32_t tiles_x) {
     NsWork w{&s, &p, first, count, ctr, tiles_x};
@@ -788,9 +788,19 @@ int cancelled(MrtContext *ctx, cudaStream_t q) {
 }
 
 // Renders of at most this many camera paths per pass run as whole-path launches, larger ones as the
-// level-by-level wavefront (MRT_PATHS_MAX; 0 = always the wavefront).  Measured on one B200: a
-// 256x256 Whitted frame 3.1x faster whole-path (launch-bound), a 512x512x4 PathTracer soup 1.2x
-// faster, a 1024x1024 terrain 1.1-1.3x slower (the wavefront's per-level coherence wins there).
+// level-by-level wavefront (MRT_PATHS_MAX; 0 = always the wavefront).  Device time of the wavefront over whole
+// paths (one B200, one light sample; Whitted to depth 4, PathTracer to depth 6, roulette beyond 3):
+//                            2^14   2^16   2^17   2^18   2^19   2^20 paths
+//   Whitted  Cornell box     4.2    4.1    3.7    2.8    2.6    1.6    (0.044 ms whole at 2^14, 0.134 at 2^19)
+//            glass room      2.8    2.8    3.0    2.4    2.1    1.5
+//            200,000 soup    1.7    1.6    1.5    1.3    1.3    1.1
+//            terrain         2.1    1.9    1.8    1.4    1.1    0.9
+//   PathTr.  Cornell box     1.0    0.8    0.6    0.4    0.3    0.2    (0.32, 2.4 ms; wavefront 0.32, 0.71)
+//            glass room      0.7    0.5    0.4    0.3    0.2    0.2
+//            200,000 soup    2.3    2.5    2.4    2.1    1.7    1.3
+//            terrain         1.9    1.8    1.7    1.3    0.9    0.6    (0.62, 2.2 ms; wavefront 1.19, 2.0)
+// The line fits open scenes and Whitted frames.  It is on the wrong side of path-traced closed rooms, whose paths
+// make five to nine rays each: the wavefront takes them from 2^14 to 2^16 paths on.
 uint64_t paths_max_setting() {
     static uint64_t v = [] {
         const char *e = getenv("MRT_PATHS_MAX");

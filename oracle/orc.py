@@ -215,6 +215,8 @@ class OrcScene:
 class RefScene:
     """The reference's own Shader::initializeAccelerators + rayTrace/shadowTrace."""
 
+    h = None
+
     def __init__(self, scene, accel: int, camera_position=None, fast: bool = False):
         self.lib = ref(fast)
         self._scene = scene
