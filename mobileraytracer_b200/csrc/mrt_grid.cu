@@ -217,8 +217,8 @@ struct WalkCells {
     uint64_t sy, sz;
     const uint32_t *start;
     // padded record i: false for the border, else the list's ends
-    __device__ bool list(uint64_t i, uint32_t &b, uint32_t &e) const {
-        const uint32_t p = G + 2u, x = (uint32_t)(i % p), y = (uint32_t)(i / p % p), z = (uint32_t)(i / ((uint64_t)p * p));
+    __device__ bool list(uint32_t i, uint32_t &b, uint32_t &e) const {
+        const uint32_t p = G + 2u, row = i / p, x = i - row * p, z = row / p, y = row - z * p;
         if (x == 0 || y == 0 || z == 0 || x > G || y > G || z > G) return false;
         const uint64_t c = (x - 1u) + (y - 1u) * sy + (z - 1u) * sz;
         b = start[c];
@@ -227,24 +227,27 @@ struct WalkCells {
     }
 };
 // reach: 0 for the border and for a cell that lists something, d for one whose surroundings are empty up to
-// d - 1 cells away
-__global__ void k_reach_init(uint64_t n, WalkCells w, uint8_t *reach) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// d - 1 cells away: the distance (of the axes' the largest) to the nearest of the former, at most kEmptyReach.
+// Axis by axis: along x, then the least over y of the larger of the steps and what x gave, then over z.
+__global__ void k_reach_init(uint32_t n, WalkCells w, uint8_t *reach) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t b, e;
-    if (i < n) reach[i] = w.list(i, b, e) && b == e ? 1 : 0;
+    if (i < n) reach[i] = w.list(i, b, e) && b == e ? (uint8_t)kEmptyReach : 0;
 }
-// d - 1 -> d where the cell and its 26 neighbours are at d - 1 (or at d already), in place
-__global__ void k_reach_grow(uint64_t n, int64_t p, uint32_t d, uint8_t *reach) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || reach[i] != d - 1) return;   // (the border stays 0: the cells left have all 26)
-    for (int64_t z = -1; z <= 1; ++z)
-        for (int64_t y = -1; y <= 1; ++y)
-            for (int64_t x = -1; x <= 1; ++x)
-                if (reach[(int64_t)i + x + (y + z * p) * p] < d - 1) return;
-    reach[i] = (uint8_t)d;
+// (the border's 0 ends every search before the array does.  Growing all cells by one step at a time, 27 neighbours
+// in seven passes, took 6.5 ms at G = 512)
+__global__ void k_reach_axis(uint32_t n, uint32_t stride, const uint8_t *__restrict__ in, uint8_t *__restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    uint32_t d = in[i];
+    for (uint32_t k = 1; k < d; ++k) {
+        const uint32_t at = k * stride;
+        d = min(d, max(k, min((uint32_t)in[i - at], (uint32_t)in[i + at])));
+    }
+    out[i] = (uint8_t)d;
 }
-__global__ void k_write_cells(uint64_t n, WalkCells w, const uint8_t *__restrict__ reach, uint2 *cells) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_write_cells(uint32_t n, WalkCells w, const uint8_t *__restrict__ reach, uint2 *cells) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     uint32_t b = 0, e = 0;
     const bool inside = w.list(i, b, e);
@@ -472,16 +475,20 @@ int build_grids(MrtScene *s, const float *cam_min, const float *cam_max, int gri
         g.id_mask = 0xFFFFFFFFu;
         const uint64_t padded = (uint64_t)(G + 2) * (uint64_t)(G + 2) * (uint64_t)(G + 2);
         if (st == MRT_OK) st = dev_alloc(ctx, s->grid_cells[type], sizeof(uint2) * padded);
-        if (st == MRT_OK) st = dev_alloc(ctx, reach, padded);
+        if (st == MRT_OK) st = dev_alloc(ctx, reach, 2 * padded);   // (at most 1026^3 cells)
         if (st == MRT_OK) {
             const uint32_t *start = (const uint32_t *)start_buf.ptr;
             const bool linear = grid_index == MRT_GRID_INDEX_LINEAR;
             const int64_t sy = linear ? (int64_t)G : (int64_t)1 << g.shift, sz = linear ? (int64_t)G * G : (int64_t)1 << (2 * g.shift);
             const WalkCells wc{(uint32_t)G, (uint64_t)sy, (uint64_t)sz, start};
             const uint32_t blocks = (uint32_t)((ncell + 255) / 256), pblocks = (uint32_t)((padded + 255) / 256);
-            k_reach_init<<<pblocks, 256, 0, q>>>(padded, wc, (uint8_t *)reach.ptr);
-            for (uint32_t d = 2; d <= kEmptyReach; ++d) k_reach_grow<<<pblocks, 256, 0, q>>>(padded, (int64_t)G + 2, d, (uint8_t *)reach.ptr);
-            k_write_cells<<<pblocks, 256, 0, q>>>(padded, wc, (const uint8_t *)reach.ptr, (uint2 *)s->grid_cells[type].ptr);
+            const uint32_t cells = (uint32_t)padded, row = (uint32_t)G + 2u;
+            uint8_t *r[2] = {(uint8_t *)reach.ptr, (uint8_t *)reach.ptr + padded};
+            k_reach_init<<<pblocks, 256, 0, q>>>(cells, wc, r[0]);
+            k_reach_axis<<<pblocks, 256, 0, q>>>(cells, 1u, r[0], r[1]);
+            k_reach_axis<<<pblocks, 256, 0, q>>>(cells, row, r[1], r[0]);
+            k_reach_axis<<<pblocks, 256, 0, q>>>(cells, row * row, r[0], r[1]);
+            k_write_cells<<<pblocks, 256, 0, q>>>(cells, wc, r[1], (uint2 *)s->grid_cells[type].ptr);
             if (type == kTriangle && n <= 1u << kSkipShift) {
                 k_skip_bits<<<blocks, 256, 0, q>>>((int64_t)ncell, sy, sz, start, (uint32_t *)s->grid_refs[type].ptr);
                 g.id_mask = (1u << kSkipShift) - 1u;
