@@ -1118,7 +1118,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
             for (int k = 0; k < 2 && st == MRT_OK; ++k)
                 if (bytes[k])
                     st = cuda_status(ctx, cudaMemcpyAsync(attempt ? own[k] : kept[k], attempt ? kept[k] : own[k], bytes[k],
-                                                          cudaMemcpyDeviceToDevice, q), "pixels kept");
+                                                          cudaMemcpyDefault, q), "pixels kept");
             if (st != MRT_OK) return st;
         }
         if (pipes == 2) {
