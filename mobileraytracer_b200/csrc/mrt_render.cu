@@ -633,7 +633,7 @@ struct TaskPlan {
     bool uploaded = false;               // explicit list already in the scene's work[0]
     bool implicit = true;
     uint32_t n_tasks = 0;
-    size_t end = 0;                      // bitmap pixels up to the last task's
+    size_t end = 0;                          // bitmap pixels up to the last task's
     std::vector<uint2> list;                 // explicit tasks (x, y) by round
     std::vector<uint32_t> next_visit;        // the same pixel's task in the next round (kNoTask: none)
     std::vector<uint32_t> round_first, round_count;
@@ -811,10 +811,11 @@ uint64_t paths_max_setting() {
 
 constexpr uint32_t kPairedRoots = 1u << 19;   // paths from which a wavefront runs as two waves at once
 
-// Paths in flight of a wavefront render: 2^22 where their queues (9.1 GB at depth 6, a quarter of it room to
-// grow) take at most an eighth of the memory that is free without them, 2^21 otherwise and on an arena, whose owner has sized it (MRT_WAVE_ROOTS: that
-// many).  Larger waves pay fewer tails and launches: the 1024x1024x16 terrain PathTracer takes 39.1 ms at
-// 2^20, 31.2 at 2^21, 27.3 at 2^22, 25.8 at 2^23 (18 GB, whose first allocation costs more than it gives).
+// Paths in flight of a wavefront render: 2^22 where their queues (7.3 GB at depth 6, allocated with a quarter
+// more to grow into) take at most an eighth of the memory that is free without them, 2^21 otherwise and on an
+// arena, whose owner has sized it (MRT_WAVE_ROOTS: that many).  Larger waves pay fewer tails and launches: the
+// 1024x1024x16 terrain PathTracer takes 39.1 ms at 2^20, 31.2 at 2^21, 27.3 at 2^22, 25.8 at 2^23 (18 GB, whose
+// first allocation costs more than it gives).
 constexpr uint32_t kWaveRoots = 1u << 21;
 uint32_t wave_roots_setting() {
     static uint32_t v = [] {
@@ -1043,7 +1044,8 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         // with more paths than that, whose tasks come tile by tile, go on with waves of half the size each time.
         int pipes = 1;
         bool pair = !paths && attempt == 0, deal = false;
-        const size_t keep_bitmap = (4 * plan.end + 255) & ~(size_t)255, keep_sums = d_accum ? 16ull * o->width * o->height : 0;
+        const size_t keep_bitmap = (4 * plan.end + 255) & ~(size_t)255;
+        const size_t keep_sums = d_accum ? 16ull * o->width * o->height : 0;
         uint32_t wave = 0;
         uint64_t ray_cap = 0, shadow_cap = 0;
         size_t queue_bytes[3] = {0, 0, 0};   // of ctx->wave[1 .. 3]
@@ -1194,7 +1196,7 @@ static int render_impl(MrtScene *s, const MrtCamera *cam, const MrtRenderOpts *o
         rays_shadow = ctx->status->count[1];
     }
     float ms = 0.0f;
-    cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
+    if (stats) cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
     if (st == MRT_ERR_LIMIT && again) {
         st = render_impl(s, cam, o, d_bitmap, stride, d_accum, stats, strata, out, attempt + 1);
         if (stats && st == MRT_OK) {
